@@ -19,6 +19,7 @@
     X(cuFuncSetAttribute, CUresult (*)(CUfunction, CUfunction_attribute, int))                    \
     X(cuLaunchKernel, CUresult (*)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned,  \
                                    unsigned, unsigned, CUstream, void **, void **))               \
+    X(cuOccupancyMaxActiveClusters, CUresult (*)(int *, CUfunction, const CUlaunchConfig *))       \
     X(cuLaunchKernelEx, CUresult (*)(const CUlaunchConfig *, CUfunction, void **, void **))       \
     X(cuMemAlloc_v2, CUresult (*)(CUdeviceptr *, size_t))                                         \
     X(cuMemFree_v2, CUresult (*)(CUdeviceptr))                                                    \

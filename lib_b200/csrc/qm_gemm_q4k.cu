@@ -1,10 +1,8 @@
-// qm_gemm_q4k.cu — prefill / batched matmul over Q4_K weights on the sm_100a tensor cores:
-// C[m][n] = sum_k A[m][k] * W[n][k], A bf16 activations, W dequantized on the fly, fp32 out.
+// qm_gemm_q4k.cu — grouped gate|up matmul of a mixture-of-experts layer that gathers its activation rows itself
+// (QM_MOE_FOLD=1): h[p][n] = silu(gate) * up over the tokens the dispatch list names, Q4_K weights dequantized on the
+// fly, bf16 activations, bf16 out. All other matmuls run in qm_gemm_pair.cu.
 //
-// Supersedes the reference's fp16 wmma 256-row "prefill" GEMM
-// (nvidia/x/cudamoe/prefill.go:97-121), which is neither quantized nor tcgen05.
-//
-// One CTA computes a 128 (weight rows) x BN (tokens, 64..512) tile of C^T:
+// One CTA computes 128 gate rows and their 128 up rows for BN tokens of one expert:
 //   * warps 2..17 form four groups of 128 threads; group g handles the K chunks g, g+4, ...: one
 //     thread per weight row reads the row's 32 quant bytes of a 64-column K chunk from the tiled
 //     weight store, turns the nibbles into exact bf16 integers with the magic-number trick (byte
@@ -12,19 +10,14 @@
 //     per pair, and writes the row into shared memory in the canonical K-major 128-byte-swizzled
 //     layout of tcgen05 (A operand); four chunks in flight hide the latency of that chain
 //     (each stage has two release barriers, so four groups may run ahead of two or three stages);
-//   * warp 0 streams the matching 64 x BN activation chunk with 2-D TMA tile copies
-//     (SWIZZLE_128B, no multicast; only the boxes that hold rows of the tile) that complete on an
-//     mbarrier (B operand) — or, for a grouped launch given the dispatch list instead of gathered
-//     rows, with tile::gather4 copies of four token rows each;
-//   * one elected thread of warp 1 issues four tcgen05.mma.kind::f16 (K = 16 each) per chunk
-//     and per 256 tokens into a TMEM accumulator of BN fp32 columns (BN = 512 uses the whole
-//     tensor memory: the dequantized tile then feeds two MMAs; N = the tile's tokens rounded up to
-//     16), tcgen05.commit frees the stage;
-//   * after the last chunk warps 2..17 read the accumulator back with tcgen05.ld (16 columns at a
-//     time, dealt evenly to the four warps of a lane quarter) and store C.
-// A ring of 2..8 shared-memory stages decouples the three roles. Every mbarrier wait is
-// bounded (qm_pipe.cuh); on expiry the status word gets QM_STATUS_TIMEOUT, the roles leave
-// their loops, TMEM is freed and the kernel returns.
+//   * warp 0 fetches the matching 64 x BN activation chunk with tile::gather4 copies of four token
+//     rows each, named by the dispatch list (B operand; bound by the rate of these copies, about
+//     26 ns each per SM);
+//   * one elected thread of warp 1 issues four tcgen05.mma.kind::f16 (K = 16 each) per chunk and
+//     sub-tile into TMEM accumulators (N = the tile's tokens rounded up to 16), tcgen05.commit
+//     frees the stage;
+//   * after the last chunk warps 2..17 read gate and up back with tcgen05.ld (16 columns at a
+//     time, dealt evenly to the four warps of a lane quarter) and store bf16 silu(gate) * up.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -71,12 +64,6 @@ __device__ __forceinline__ uint32_t bf2(float v) {   // (v, v) as bf16x2
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(tmap), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
 // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart (sm_100 descriptor version 1)
 // Four rows (y0..y3) of a 2-D tensor, box columns starting at x, into four consecutive rows at dst.
 __device__ __forceinline__ void tma_gather4(uint32_t dst, const void *tmap, int x, int y0, int y1, int y2, int y3,
@@ -102,11 +89,8 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 
 }  // namespace
 
-// NSUB = 128-row sub-tiles of weight rows per CTA: 1 (128 x BN tile, BN up to 512) or 2
-// (256 x BN tile, BN up to 256: half the activation traffic per flop and room for a third stage).
-// KS = 64-column K chunks per pipeline stage: 1, or 2 for small token tiles, where the barrier
-// handshake of a stage (about 0.3 us, whatever the stage count) is longer than the MMAs of one
-// chunk: two chunks per handshake halve it.
+// KS = 64-column K chunks per pipeline stage: 1, or 2 where two such stages fit (the barrier handshake of a stage,
+// about 0.3 us whatever the stage count, is longer than the MMAs of one small chunk).
 #ifdef QM_DEBUG
 __device__ __forceinline__ unsigned long long gtime() {
     unsigned long long t;
@@ -115,7 +99,7 @@ __device__ __forceinline__ unsigned long long gtime() {
 }
 #define QM_GEMM_STAMP(i)                                                                                       \
     do {                                                                                                       \
-        if ((a.debug & 64) && a.swiglu) {                                                                      \
+        if (a.debug & 64) {                                                                      \
             const int L_ = blockIdx.y * gridDim.x + blockIdx.x;                                                \
             if (L_ < 990) reinterpret_cast<unsigned long long *>(a.status + 256)[L_ * 4 + (i)] = gtime();      \
         }                                                                                                      \
@@ -124,8 +108,9 @@ __device__ __forceinline__ unsigned long long gtime() {
 #define QM_GEMM_STAMP(i)
 #endif
 
-template <int NSUB, int KS>
+template <int KS>
 __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
+    constexpr int NSUB = 2;   // 128-row sub-tiles: gate rows and the up rows that belong to them
     extern __shared__ uint8_t smem_raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) QM_GEMM_STAMP(0);
@@ -151,32 +136,17 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
     };
     const uint32_t smem_base = smem_u32(smem);
 
-    const bool fuse_swiglu = NSUB == 2 && a.swiglu != 0;
-    // grouped launches put the expert in blockIdx.y and the token tile in blockIdx.z: CTAs are
-    // handed out x-fastest, then y, then z, so every expert's first token tiles (the ones with
-    // work) start before the mostly empty later tiles
-    // (grouped launches with split K: blockIdx.z = token tile * splitk + K share)
-    const int n0 = blockIdx.x * kBM * (fuse_swiglu ? 1 : NSUB), m0 = (a.grouped ? (int)blockIdx.z / a.splitk : (int)blockIdx.y) * BN;
-    // grouped launch: this CTA's expert, its rows of the gathered activations and its weights
-    int row_off = 0, m_cnt = a.m;
-    const uint8_t *wq = a.wq;
-    if (a.grouped) {
-        const int e = blockIdx.y;
-        row_off = a.offsets[e];
-        m_cnt = a.offsets[e + 1] - row_off;
-        if (m0 >= m_cnt) return;   // nothing routed here (uniform over the CTA, before any barrier)
-        wq = a.wq_list[e];
-    }
-    // 64-column chunks along K; with split K (splitk > 1) this CTA takes a contiguous share
-    // and stores its partial tile to its own plane of the scratch (added up in a fixed order at the end)
-    const int nk_all = a.units * 4 / KS;      // stage chunks of KS x 64 columns
-    const int zk = a.grouped ? (int)blockIdx.z % a.splitk : (int)blockIdx.z;
-    const int kc_lo = (int)((int64_t)nk_all * zk / a.splitk);
-    const int nk = (int)((int64_t)nk_all * (zk + 1) / a.splitk) - kc_lo;
+    // the expert is in blockIdx.y and the token tile in blockIdx.z: CTAs are handed out x-fastest, then y, then z, so
+    // every expert's first token tiles (the ones with work) start before the mostly empty later tiles
+    const int n0 = blockIdx.x * kBM, m0 = (int)blockIdx.z * BN;
+    const int row_off = a.offsets[blockIdx.y], m_cnt = a.offsets[blockIdx.y + 1] - row_off;
+    if (m0 >= m_cnt) return;   // nothing routed here (uniform over the CTA, before any barrier)
+    const uint8_t *wq = a.wq_list[blockIdx.y];
+    const int nk = a.units * 4 / KS;          // stage chunks of KS x 64 columns
 
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) {
-            mbar_init(full_a + 8 * s, a.groups == 4 ? 4 : 8);   // warps of one producer group
+            mbar_init(full_a + 8 * s, 4);   // warps of one producer group
             mbar_init(full_b + 8 * s, 1);
             mbar_init(empty + 8 * (2 * s), 1);
             mbar_init(empty + 8 * (2 * s + 1), 1);
@@ -198,7 +168,7 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && a.gather_list) {
+    if (warp == 0) {
         // ---- activation chunks gathered by the rows' token numbers ----------------------------
         // One tile::gather4 copy brings the 64-column chunk of four rows named by their row numbers
         // in the tokens' own matrix (a tensor map with a one-row box) into four consecutive
@@ -220,25 +190,8 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
                 for (int g4 = lane; g4 < BN / 4; g4 += 32) {
                     const int4 t = *reinterpret_cast<const int4 *>(tok + 4 * g4);
                     tma_gather4(smem_base + s * stage_bytes + a_bytes + j * b_tile + g4 * 512, &a.tmap_gather,
-                                ((kc_lo + kc) * KS + j) * kBK, t.x, t.y, t.z, t.w, full_b + 8 * s);
+                                (kc * KS + j) * kBK, t.x, t.y, t.z, t.w, full_b + 8 * s);
                 }
-        }
-    } else if (warp == 0) {
-        // ---- activation chunks by TMA ---------------------------------------------------------
-        if (lane == 0) {
-            const int box = a.box_rows, nbox = (min(BN, m_cnt - m0) + box - 1) / box;
-            for (int kc = 0; kc < nk; kc++) {
-                const int s = kc % kStages;
-                if (!wait_empty(kc)) { atomicOr(a.status, QM_STATUS_TIMEOUT); break; }
-                if (QM_GEMM_DEBUG_BIT(2)) { mbar_arrive(full_b + 8 * s); continue; }
-                // only the boxes that hold rows of this tile (an MMA reads no further than its N)
-                mbar_expect_tx(full_b + 8 * s, (uint32_t)(KS * nbox * box * 128));
-#pragma unroll
-                for (int j = 0; j < KS; j++)
-                    for (int nb = 0; nb < nbox * box; nb += box)   // a TMA box has at most 256 rows
-                        tma_load_2d(smem_base + s * stage_bytes + a_bytes + j * b_tile + nb * 128, &a.tmap_act,
-                                    ((kc_lo + kc) * KS + j) * kBK, row_off + m0 + nb, full_b + 8 * s);
-            }
         }
     } else if (warp == 1) {
         // ---- MMA issue ----------------------------------------------------------------------------
@@ -283,17 +236,15 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
         // chunk into its 64 bf16 columns. A thread's iteration is a chain of dependent steps (wait
         // for the stage, convert, store, fence, arrive); four chunks in flight hide that latency.
         // With fewer stages than groups a group's loads are in flight while it waits for a stage.
-        // (Two groups — two threads per row, one per nibble half — is the other form the host can ask for.)
-        const int kGroups = a.groups == 4 ? 4 : 2;
+        constexpr int kGroups = 4;
         const int pt = tid - 64;
         const int r = pt & 127;              // row of a 128-row sub-tile
-        const int grp = kGroups == 4 ? pt >> 7 : pt >> 8;   // warp-uniform
-        const int my_hs = kGroups == 4 ? -1 : (pt >> 7) & 1;   // the nibble half of this thread, or both
+        const int grp = pt >> 7;             // warp-uniform
         const int rr = (n0 + r) & 15;
         const uint8_t *row_items[NSUB];
 #pragma unroll
         for (int sub = 0; sub < NSUB; sub++) {
-            const int sub_row = fuse_swiglu ? sub * a.up_offset : sub * kBM;   // up rows sit up_offset below the gate rows
+            const int sub_row = sub * a.up_offset;   // up rows sit up_offset below the gate rows
             const int64_t tile16 = min((n0 + sub_row + r) >> 4, a.tiles16 - 1);
             row_items[sub] = wq + tile16 * a.units * QM_Q4K_ITEM_BYTES;
         }
@@ -312,7 +263,7 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
             if (QM_GEMM_DEBUG_BIT(8)) return;
 #pragma unroll
             for (int j = 0; j < KS; j++) {
-                const int c64 = (kc_lo + kcl) * KS + j;   // 64-column chunk along K
+                const int c64 = kcl * KS + j;   // 64-column chunk along K
 #pragma unroll
                 for (int sub = 0; sub < NSUB; sub++) {
                     const uint8_t *item = row_items[sub] + (size_t)(c64 >> 2) * QM_Q4K_ITEM_BYTES;
@@ -328,7 +279,7 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
             if (!wait_empty(kc)) { atomicOr(a.status, QM_STATUS_TIMEOUT); ok = false; break; }
 #pragma unroll
             for (int j = 0; j < KS; j++) {
-                const int p = ((kc_lo + kc) * KS + j) & 3;
+                const int p = (kc * KS + j) & 3;
 #pragma unroll
                 for (int sub = 0; sub < NSUB; sub++) {
                     if (QM_GEMM_DEBUG_BIT(1)) break;
@@ -357,7 +308,6 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
                     uint8_t *arow = smem + (size_t)s * stage_bytes + j * a_tile + sub * kATile + r * 128;
 #pragma unroll
                     for (int hs = 0; hs < 2; hs++) {
-                        if (my_hs >= 0 && hs != my_hs) continue;
 #pragma unroll
                         for (int c = 0; c < 4; c++) {   // 16-byte pieces (eight columns), XOR-swizzled by the row inside its 8-row group
                             uint32_t o[4];
@@ -398,50 +348,22 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
                     : "memory");
             };
             const uint32_t quarter_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);   // TMEM lane quarter of this warp
-            if (fuse_swiglu) {
-                // gate in accumulator 0, the matching up rows in accumulator 1: h = silu(gate) * up
-                const int n = n0 + (warp & 3) * 32 + lane;
-                for (int c0 = cbeg; c0 < cend; c0 += 16) {
-                    uint32_t g[16], u[16];
-                    tmem_ld16(quarter_base + (uint32_t)c0, g);
-                    tmem_ld16(quarter_base + (uint32_t)(BN + c0), u);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (n < a.n) {
-                        uint16_t *hp = a.h + (int64_t)(row_off + m0 + c0) * a.ldh + n;
+            // gate in accumulator 0, the matching up rows in accumulator 1: h = silu(gate) * up
+            const int n = n0 + (warp & 3) * 32 + lane;
+            for (int c0 = cbeg; c0 < cend; c0 += 16) {
+                uint32_t g[16], u[16];
+                tmem_ld16(quarter_base + (uint32_t)c0, g);
+                tmem_ld16(quarter_base + (uint32_t)(BN + c0), u);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (n < a.n) {
+                    uint16_t *hp = a.h + (int64_t)(row_off + m0 + c0) * a.ldh + n;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            if (m0 + c0 + j < m_cnt) {
-                                const float gv = __uint_as_float(g[j]), uv = __uint_as_float(u[j]);
-                                // (fast division: the quotient is rounded to bf16 next; the IEEE form cost 10 us per CTA here)
-                                const __nv_bfloat16 hv = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
-                                hp[(int64_t)j * a.ldh] = *reinterpret_cast<const uint16_t *>(&hv);
-                            }
-                        }
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int sub = 0; sub < NSUB; sub++) {
-                    const int n = n0 + sub * kBM + (warp & 3) * 32 + lane;
-                    // split K: this CTA's share of the tile goes to its own plane of the scratch
-                    float *base = a.splitk == 1 ? a.c : a.partials + (int64_t)zk * a.plane_rows * a.n;
-                    const int64_t ld = a.splitk == 1 ? a.ldc : a.n;
-                    for (int c0 = cbeg; c0 < cend; c0 += 32) {   // two blocks per wait where there are two
-                        uint32_t v[16], w[16];
-                        const bool two = c0 + 16 < cend;
-                        tmem_ld16(quarter_base + (uint32_t)(sub * BN + c0), v);
-                        if (two) tmem_ld16(quarter_base + (uint32_t)(sub * BN + c0 + 16), w);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (n < a.n) {
-                            float *cp = base + (int64_t)(row_off + m0 + c0) * ld + n;
-#pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                if (m0 + c0 + j < m_cnt) cp[(int64_t)j * ld] = __uint_as_float(v[j]);
-                            if (two) {
-#pragma unroll
-                                for (int j = 0; j < 16; j++)
-                                    if (m0 + c0 + 16 + j < m_cnt) cp[(int64_t)(16 + j) * ld] = __uint_as_float(w[j]);
-                            }
+                    for (int j = 0; j < 16; j++) {
+                        if (m0 + c0 + j < m_cnt) {
+                            const float gv = __uint_as_float(g[j]), uv = __uint_as_float(u[j]);
+                            // (fast division: the quotient is rounded to bf16 next; the IEEE form cost 10 us per CTA here)
+                            const __nv_bfloat16 hv = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
+                            hp[(int64_t)j * a.ldh] = *reinterpret_cast<const uint16_t *>(&hv);
                         }
                     }
                 }
@@ -457,85 +379,12 @@ __device__ __forceinline__ void gemm_body(const QmGemmArgs &a) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
-    if (a.splitk > 1) {
-        // Every CTA of the tile adds one band of it, in order of z, once all splitk shares are in the scratch:
-        // the launch is cooperative (all CTAs resident), the wait for the others is bounded. (The barrier
-        // above ordered every thread's stores before thread 0's fence and arrival.)
-        volatile uint32_t *s_ok = tmem_slot + 1;   // a free word of the dynamic shared memory's tail
-        const unsigned int tile_id = a.grouped ? ((blockIdx.z / a.splitk) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x
-                                               : blockIdx.y * gridDim.x + blockIdx.x;
-        unsigned int *ticket = a.tickets + 2 * tile_id;
-        if (tid == 0) {
-            __threadfence();
-            atomicAdd(ticket, 1u);
-            const long long t0 = clock64();
-            bool ok = true;
-            while (ld_acquire(ticket) < (unsigned int)a.splitk) {
-                if (clock64() - t0 > a.wait_cycles) { atomicOr(a.status, QM_STATUS_TIMEOUT); ok = false; break; }
-            }
-            *s_ok = ok ? 1u : 0u;
-        }
-        __syncthreads();
-        if (*s_ok) {
-            const int rows = min(NSUB * kBM, a.n - n0), toks = min(BN, m_cnt - m0);
-            const int t_lo = (int)((int64_t)toks * zk / a.splitk) + row_off, t_hi = (int)((int64_t)toks * (zk + 1) / a.splitk) + row_off;
-            const int64_t plane = (int64_t)a.plane_rows * a.n;
-            if ((rows & 3) == 0 && (a.n & 3) == 0 && (a.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(a.c) & 15) == 0) {
-                // 16 bytes per thread and four of them in flight: the loop is bound by the latency of its loads
-                const int r4 = rows >> 2, total = r4 * (t_hi - t_lo), step = (int)blockDim.x;
-                for (int i0 = tid; i0 < total; i0 += 4 * step) {
-                    float4 acc[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int i = i0 + u * step;
-                        acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (i < total) {
-                            const int mm = t_lo + i / r4, nn = (i % r4) << 2;
-                            const float *src = a.partials + (int64_t)(m0 + mm) * a.n + n0 + nn;
-                            for (int z = 0; z < a.splitk; z++) {
-                                const float4 v = __ldcg(reinterpret_cast<const float4 *>(src + z * plane));
-                                acc[u].x += v.x; acc[u].y += v.y; acc[u].z += v.z; acc[u].w += v.w;
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int i = i0 + u * step;
-                        if (i < total) {
-                            const int mm = t_lo + i / r4, nn = (i % r4) << 2;
-                            *reinterpret_cast<float4 *>(a.c + (int64_t)(m0 + mm) * a.ldc + n0 + nn) = acc[u];
-                        }
-                    }
-                }
-            } else {
-                for (int i = tid; i < rows * (t_hi - t_lo); i += blockDim.x) {
-                    const int mm = t_lo + i / rows, nn = i % rows;
-                    const int64_t at = (int64_t)(m0 + mm) * a.n + n0 + nn;
-                    float sum = 0.f;
-                    for (int z = 0; z < a.splitk; z++) sum += __ldcg(a.partials + z * plane + at);
-                    a.c[(int64_t)(m0 + mm) * a.ldc + n0 + nn] = sum;
-                }
-            }
-        }
-        // the last CTA to finish its band zeroes the tile's two words for the next launch
-        __syncthreads();
-        if (tid == 0 && atomicAdd(ticket + 1, 1u) + 1u == (unsigned int)a.splitk) {
-            ticket[0] = 0u;
-            ticket[1] = 0u;
-        }
-    }
 }
 
-extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_bf16(const __grid_constant__ QmGemmArgs a) {
-    gemm_body<1, 1>(a);
+extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_gather(const __grid_constant__ QmGemmArgs a) {
+    gemm_body<1>(a);
 }
-extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_bf16_r256(const __grid_constant__ QmGemmArgs a) {
-    gemm_body<2, 1>(a);
-}
-// Two 64-column chunks per stage (small token tiles).
-extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_bf16_k128(const __grid_constant__ QmGemmArgs a) {
-    gemm_body<1, 2>(a);
-}
-extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_bf16_r256_k128(const __grid_constant__ QmGemmArgs a) {
-    gemm_body<2, 2>(a);
+// Two 64-column chunks per stage.
+extern "C" __global__ void __launch_bounds__(576, 1) qm_gemm_q4k_gather_k128(const __grid_constant__ QmGemmArgs a) {
+    gemm_body<2>(a);
 }

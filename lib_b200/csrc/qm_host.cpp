@@ -55,6 +55,7 @@ QM_INCBIN(qm_cubin_gemv, QM_STR(QM_CUBIN_DIR) "/qm_gemv.sm_100a.cubin")
 QM_INCBIN(qm_cubin_dequant, QM_STR(QM_CUBIN_DIR) "/qm_dequant.sm_100a.cubin")
 QM_INCBIN(qm_cubin_q4k, QM_STR(QM_CUBIN_DIR) "/qm_gemv_q4k.sm_100a.cubin")
 QM_INCBIN(qm_cubin_gemm, QM_STR(QM_CUBIN_DIR) "/qm_gemm_q4k.sm_100a.cubin")
+QM_INCBIN(qm_cubin_pair, QM_STR(QM_CUBIN_DIR) "/qm_gemm_pair.sm_100a.cubin")
 QM_INCBIN(qm_cubin_moe, QM_STR(QM_CUBIN_DIR) "/qm_moe.sm_100a.cubin")
 QM_INCBIN(qm_cubin_kq, QM_STR(QM_CUBIN_DIR) "/qm_gemv_kq.sm_100a.cubin")
 QM_INCBIN(qm_cubin_q81, QM_STR(QM_CUBIN_DIR) "/qm_q8_1.sm_100a.cubin")
@@ -68,6 +69,7 @@ static const KernelImage kImages[QM_MOD_COUNT] = {
     {qm_cubin_dequant, qm_cubin_dequant_end},
     {qm_cubin_q4k, qm_cubin_q4k_end},
     {qm_cubin_gemm, qm_cubin_gemm_end},
+    {qm_cubin_pair, qm_cubin_pair_end},
     {qm_cubin_moe, qm_cubin_moe_end},
     {qm_cubin_kq, qm_cubin_kq_end},
     {qm_cubin_q81, qm_cubin_q81_end},
@@ -90,8 +92,8 @@ static const KernelName kKernels[QM_K_COUNT] = {
     {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d2_tp"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d3_tp"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d4_tp"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d2_tp"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d3_tp"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d4_tp"},
     {QM_MOD_Q4K, "qm_sum_parts"}, {QM_MOD_DEQUANT, "qm_repack_parts"},
-    {QM_MOD_GEMM, "qm_gemm_q4k_bf16"}, {QM_MOD_GEMM, "qm_gemm_q4k_bf16_r256"},
-    {QM_MOD_GEMM, "qm_gemm_q4k_bf16_k128"}, {QM_MOD_GEMM, "qm_gemm_q4k_bf16_r256_k128"},
+    {QM_MOD_GEMM, "qm_gemm_q4k_gather"}, {QM_MOD_GEMM, "qm_gemm_q4k_gather_k128"},
+    {QM_MOD_PAIR, "qm_gemm_q4k_pair"}, {QM_MOD_PAIR, "qm_gemm_q4k_solo"},
     {QM_MOD_MOE, "qm_moe_route"},      {QM_MOD_MOE, "qm_moe_lists"},      {QM_MOD_MOE, "qm_moe_gather"},
     {QM_MOD_MOE, "qm_moe_combine"},
     {QM_MOD_DEQUANT, "qm_dequant_iq2xxs"},
@@ -197,10 +199,8 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
         if (!err) {
-            r = d->cuFuncSetAttribute(c->fn[QM_K_GEMM_Q4K], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
-            for (int k = QM_K_GEMM_Q4K_R256; k <= QM_K_GEMM_Q4K_R256_K128 && r == CUDA_SUCCESS; k++)
+            for (int k = QM_K_GEMM_GATHER; k <= QM_K_GEMM_SOLO && r == CUDA_SUCCESS; k++)
                 r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
-
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
         for (int k = QM_K_FUSED_Q4K_DD_N2D2; k <= QM_K_FUSED_Q4K_DD_N2D3 && !err; k++) {
@@ -223,6 +223,9 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
+        for (int cg = 1; cg <= 2 && !err; cg++)
+            for (int k = 1; k <= 4; k *= 2)
+                c->gemm_clusters[cg - 1][k] = qm_max_clusters(c, cg == 2 ? QM_K_GEMM_PAIR : QM_K_GEMM_SOLO, cg * k, 768, QM_GEMV_SMEM_MAX);
         if (!err) {
             r = d->cuStreamCreate(&c->own_stream, CU_STREAM_NON_BLOCKING);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
@@ -360,7 +363,7 @@ extern "C" int32_t qm_memcpy_d2h(qm_ctx *c, void *dst, uint64_t src, int64_t byt
 
 // ---- launch helper ----------------------------------------------------------------------
 static int32_t launch_grid(qm_ctx *c, int kernel, unsigned gx, unsigned gy, unsigned block, unsigned smem, void *args,
-                           bool pdl, bool cooperative) {
+                           bool pdl, bool cooperative, int cluster = 1) {
     void *params[1] = {args};
     CUlaunchConfig cfg;
     memset(&cfg, 0, sizeof cfg);
@@ -372,8 +375,14 @@ static int32_t launch_grid(qm_ctx *c, int kernel, unsigned gx, unsigned gy, unsi
     cfg.blockDimZ = 1;
     cfg.sharedMemBytes = smem;
     cfg.hStream = c->stream;
-    CUlaunchAttribute attr[2];
+    CUlaunchAttribute attr[3];
     unsigned n = 0;
+    if (cluster > 1) {
+        attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+        attr[n].value.clusterDim.x = (unsigned)cluster;
+        attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
+        n++;
+    }
     if (pdl) {
         attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
         attr[n].value.programmaticStreamSerializationAllowed = 1;
@@ -392,8 +401,27 @@ static int32_t launch_grid(qm_ctx *c, int kernel, unsigned gx, unsigned gy, unsi
 }
 
 int32_t qm_launch_ex(qm_ctx *c, int kernel, unsigned gx, unsigned block, unsigned smem, void *args, bool pdl,
-                     bool cooperative) {
-    return launch_grid(c, kernel, gx, 1, block, smem, args, pdl, cooperative);
+                     bool cooperative, int cluster) {
+    return launch_grid(c, kernel, gx, 1, block, smem, args, pdl, cooperative, cluster);
+}
+
+int qm_max_clusters(qm_ctx *c, int kernel, int cluster, unsigned block, unsigned smem) {
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDimX = (unsigned)cluster;
+    cfg.gridDimY = cfg.gridDimZ = 1;
+    cfg.blockDimX = block;
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = smem;
+    cfg.hStream = c->stream;
+    CUlaunchAttribute attr;
+    attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+    attr.value.clusterDim.x = (unsigned)cluster;
+    attr.value.clusterDim.y = attr.value.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    return c->drv->cuOccupancyMaxActiveClusters(&n, c->fn[kernel], &cfg) == CUDA_SUCCESS ? n : 0;
 }
 
 int32_t qm_launch(qm_ctx *c, int kernel, unsigned gx, unsigned gy, unsigned block, unsigned smem, void *args,
@@ -1015,49 +1043,75 @@ extern "C" int32_t qm_matvec_host(qm_ctx *c, qm_weight h, const float *x_host, i
     return QM_OK;
 }
 
-// ---- prefill matmul (tcgen05) ----------------------------------------------------------------
-// One launch of the tcgen05 matmul. Single matrix: g.experts == 0, weights w, activations
-// a_dev [m][lda]. Grouped over experts (g.experts > 0): blockIdx.z = expert, its activation rows
-// are [offsets[e], offsets[e+1]) of a_dev [rows_total][lda], its weights wq_list[e] (all experts
-// shaped like w); m = the longest expert list (sizes the grid). With g.swiglu the weights are
-// gate|up matrices [2*ffn][k] and the launch stores bf16 silu(gate)*up to g.h instead of C.
-int32_t qm_gemm_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
-                       uint64_t c_dev, int64_t ldc, const QmGemmGroup &g) {
-    QmGemmArgs a;
+// ---- matmul by CTA pairs ----------------------------------------------------------------------
+// The tile of a pair launch: CTAs per tile, tokens per tile, K shares per tile (one cluster).
+struct QmPairPlan {
+    int cg, bn, splitk;
+};
+
+// Estimated cycles: a stage of 128 columns takes 4 cycles per token column on the tensor cores (a CTA alone also copies
+// and reads all of B: 6), at least what its dequantization and hand-over take; a tile's accumulator read-out is hidden
+// by the next tile only where two accumulators fit.
+static QmPairPlan plan_pair(const qm_ctx *c, int64_t rows, int64_t m, int units) {
+    QmPairPlan best = {2, 64, 1};
+    double best_cost = 0;
+    for (int cg = 1; cg <= 2; cg++)
+        for (int bn = 32; bn <= 256; bn += 32) {
+            const int64_t tiles = (rows + 128 * cg - 1) / (128 * cg) * ((m + bn - 1) / bn);
+            for (int s = 1; s * cg <= 4; s *= 2) {   // clusters of up to four CTAs (of eight only 15 fit at once)
+                const int at_once = c->gemm_clusters[cg - 1][s];
+                if (at_once < 1 || (s > 1 && (tiles > at_once || units < s))) continue;
+                const int64_t rounds = (tiles + at_once - 1) / at_once;
+                const double stage = std::max((cg == 2 ? 4.0 : 5.0) * bn, 500.0), readout = 12.0 * bn + (s > 1 ? 2000 : 0);
+                const double cost = rounds * (units * 2.0 / s * stage + 500) + (bn <= 128 ? readout : rounds * readout);
+                if (best_cost == 0 || cost < best_cost) {
+                    best = {cg, bn, s};
+                    best_cost = cost;
+                }
+            }
+        }
+    return best;
+}
+
+static int32_t pair_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
+                           uint64_t c_dev, int64_t ldc, const QmGemmGroup &g) {
+    QmPairArgs a;
     memset(&a, 0, sizeof a);
     const bool grouped = g.experts > 0;
-    // Tile shapes: 128 weight rows x 64..512 tokens per CTA (four stages, two at 512 tokens). A
-    // 256-row variant (two accumulators, three or four stages) serves the fused SwiGLU epilogue
-    // (gate rows in one accumulator, the matching up rows in the other); for plain matmuls it is
-    // kept behind QM_GEMM_R256=1: measured equal within noise (76.6 us against 74.0 us at
-    // 4096 x 4096 x 2048), so neither the stage count nor the activation traffic is the limit.
-    const int mt = g.m_typical > 0 ? g.m_typical : m;
-    // ... and the grouped down launch where 128-row tiles would not fit one wave of the SMs (eight experts
-    // of 4096 rows: 256 tiles are 1.73 waves, 128 tiles of 256 rows are one; MoE layer 0.647 -> 0.612 ms)
-    const bool r256_wave = grouped && !g.swiglu && mt <= 256 && w->rows >= 256 &&
-                           ((w->rows + 127) / 128) * (int64_t)g.experts > c->sm_count;
-    const bool r256 = g.swiglu || (env_int("QM_GEMM_R256", r256_wave ? 1 : 0) != 0 && w->rows >= 256);
-    const int nsub = r256 ? 2 : 1;
-    // (192: a grouped launch whose longest list fits gets a smaller activation tile and with it a fourth stage)
-    const int bn_auto = mt <= 64 ? 64 : mt <= 128 ? 128 : (grouped && mt <= 192) ? 192 : (mt <= 256 || r256) ? 256 : 512;
-    const int bn = std::min(bn_auto, std::max(64, env_int("QM_GEMM_BN", 512)));
-    // Two 64-column chunks per stage where at least two such stages fit and the token tile is
-    // small: the handshake of a stage costs ~0.3 us, more than the MMAs of one small chunk.
-    const int chunk_bytes = nsub * 128 * 64 * 2 + bn * 64 * 2;
-    const int ks = env_int("QM_GEMM_KS", (bn <= 256 && (QM_GEMV_SMEM_MAX - 2048) / (2 * chunk_bytes) >= 2) ? 2 : 1) == 2 ? 2 : 1;
-    const int stage_bytes = ks * chunk_bytes;
-    const int stages = std::max(2, std::min(8, (QM_GEMV_SMEM_MAX - 2048) / stage_bytes));
-    if (stages * stage_bytes + 2048 > QM_GEMV_SMEM_MAX) return QM_ERR_SHAPE;
+    const int64_t out_cols = g.swiglu ? w->rows / 2 : w->rows;
+    QmPairPlan p;
+    if (grouped) {
+        // token tiles of equal size, at most 160 (an expert's weights are dequantized once per token tile)
+        const int mt = g.m_typical > 0 ? g.m_typical : m, nt = (mt + 159) / 160;
+        p = {2, std::max(32, ((mt + nt - 1) / nt + 31) & ~31), 1};
+        // few experts per GPU (expert-parallel runs) leave pairs idle: two of them share a tile's K
+        // (decided by the mean list, which is known also where the lists stay on the device)
+        const int64_t most = (out_cols + 255) / 256 * ((rows_total / g.experts + 159) / 160) * g.experts;
+        if (!g.swiglu && most <= c->gemm_clusters[1][2] && w->units >= 2 && env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0) p.splitk = 2;
+    } else {
+        p = plan_pair(c, out_cols, m, w->units);
+    }
+    const int tile_rows = (g.swiglu ? 64 : 128) * p.cg;
+    const int64_t row_tiles = (out_cols + tile_rows - 1) / tile_rows;
+    const int64_t tiles = row_tiles * ((m + p.bn - 1) / p.bn) * (grouped ? g.experts : 1);
+    if (!grouped && tiles * p.cg * p.splitk > (1 << 30)) return QM_ERR_SHAPE;
+    const int stage_bytes = p.bn * 256 / p.cg;
+    a.bn = p.bn;
+    a.nacc = p.bn <= 128 ? 2 : 1;
+    // (at least four units of weight items stay in flight)
+    a.stages = std::min(std::min(8, (512 - a.nacc * a.bn) / 64), (QM_GEMV_SMEM_MAX - 2560 - 4 * 8 * QM_Q4K_ITEM_BYTES) / stage_bytes);
+    a.raw_ring = std::min(8, (QM_GEMV_SMEM_MAX - 2560 - a.stages * stage_bytes) / (8 * QM_Q4K_ITEM_BYTES));
+    a.splitk = p.splitk;
+    a.row_tiles = (int32_t)row_tiles;
+    a.items = grouped ? 0 : (int32_t)tiles;   // grouped: the pairs walk the lists
+    a.box_rows = a.bn / p.cg;
     const cuuint64_t dims[2] = {(cuuint64_t)w->cols, (cuuint64_t)rows_total};
     const cuuint64_t strides[1] = {(cuuint64_t)lda * 2};
-    // grouped launches fetch the token tile in boxes of 64 rows, as many as the expert's list fills
-    const int box_rows = grouped ? 64 : std::min(bn, 256);
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {64, (cuuint32_t)a.box_rows};
     const cuuint32_t estr[2] = {1, 1};
     DRV(c->drv->cuTensorMapEncodeTiled(&a.tmap_act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)(uintptr_t)a_dev, dims,
                                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-    const int64_t out_cols = g.swiglu ? w->rows / 2 : w->rows;   // columns of the output matrix
     a.wq = (const uint8_t *)(uintptr_t)w->wq;
     a.c = (float *)(uintptr_t)c_dev;
     a.status = (unsigned int *)(uintptr_t)c->status_dev;
@@ -1066,79 +1120,102 @@ int32_t qm_gemm_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, 
     a.n = (int32_t)out_cols;
     a.units = w->units;
     a.tiles16 = (int32_t)((w->rows + 15) / 16);
-    a.bn = bn;
-    a.stages = stages;
-    a.box_rows = box_rows;
-    a.groups = env_int("QM_GEMM_GROUPS", 4) == 2 ? 2 : 4;
     a.grouped = grouped ? 1 : 0;
+    a.experts = g.experts;
     a.wq_list = (const uint8_t *const *)(uintptr_t)g.wq_list_dev;
     a.offsets = (const int32_t *)(uintptr_t)g.offsets_dev;
     a.swiglu = g.swiglu ? 1 : 0;
     a.up_offset = (int32_t)(w->rows / 2);
     a.h = (uint16_t *)(uintptr_t)g.h_dev;
     a.ldh = g.ldh;
-#ifdef QM_DEBUG
-    a.debug = env_int("QM_GEMM_DEBUG", 0);
-#endif
-    unsigned smem = 1024 + stages * stage_bytes + 512;   // alignment slack, stages, barriers
-    if (g.gather_list_dev) {   // the loader warp's table of token numbers sits behind the barriers
-        if (!grouped || bn > 256 || g.gather_topk < 1) return QM_ERR_SHAPE;
-        a.gather_list = (const int32_t *)(uintptr_t)g.gather_list_dev;
-        a.gather_topk = g.gather_topk;
-        const cuuint32_t row_box[2] = {64, 1};   // tile::gather4 names the four rows itself
-        DRV(c->drv->cuTensorMapEncodeTiled(&a.tmap_gather, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)(uintptr_t)a_dev,
-                                           dims, strides, row_box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-        smem += 1024;
-        if (smem > QM_GEMV_SMEM_MAX) return QM_ERR_SHAPE;
-    }
     void *params[1] = {&a};
     CUlaunchConfig cfg;
     memset(&cfg, 0, sizeof cfg);
-    const int rows_per_cta = g.swiglu ? 128 : 128 * nsub;
-    cfg.gridDimX = (unsigned)((out_cols + rows_per_cta - 1) / rows_per_cta);
-    cfg.gridDimY = (unsigned)((m + bn - 1) / bn);
-    // few tokens: split K over CTAs until the SMs are covered; the last CTA of a tile adds the shares in a
-    // fixed order (no atomics on C: the same bits every run)
-    int splitk = 1;
-    // (grouped launches too, where the experts' tiles leave SMs idle — few experts per GPU in expert-parallel
-    // runs; not with the SwiGLU epilogue, whose launches have row tiles enough)
-    const int64_t tiles = (int64_t)cfg.gridDimX * cfg.gridDimY * (grouped ? g.experts : 1);
-    const int64_t plane_rows = grouped ? rows_total : m;
-    if (!g.swiglu) {
-        while (splitk < 8 && tiles * splitk * 2 <= c->sm_count && w->units * 4 / (splitk * 2) >= 8) splitk *= 2;
-        if (!grouped) splitk = env_int("QM_GEMM_SPLITK", splitk);
-        else if (env_int("QM_GEMM_GROUPED_SPLITK", 1) == 0) splitk = 1;
-    }
-    // the shares go through the context's scratch (one plane of rows x n floats per share) and a ticket per tile
-    while (splitk > 1 && ((int64_t)splitk * plane_rows * out_cols * 4 > QM_PARTIALS_BYTES || tiles * 2 > QM_TICKETS))
-        splitk /= 2;
-    a.splitk = splitk;
-    a.plane_rows = (int32_t)plane_rows;
-    a.partials = (float *)(uintptr_t)c->partials_dev;
-    a.tickets = (unsigned int *)(uintptr_t)c->tickets_dev;
-    a.wait_cycles = qm_wait_cycles();
-    cfg.gridDimZ = (unsigned)splitk;
-    if (grouped) {   // expert in y, token tile and K share in z (see the kernel)
-        cfg.gridDimZ = cfg.gridDimY * (unsigned)splitk;
-        cfg.gridDimY = (unsigned)g.experts;
-    }
-    cfg.blockDimX = 576;   // TMA warp, MMA warp, sixteen dequantizing warps
+    // persistent: pair p takes the tiles p, p + pairs, ... (split K: one cluster per tile)
+    cfg.gridDimX = (unsigned)(p.cg * (p.splitk > 1 ? tiles * p.splitk : std::min<int64_t>(tiles, c->sm_count / p.cg)));
+    cfg.gridDimY = cfg.gridDimZ = 1;
+    cfg.blockDimX = 768;
     cfg.blockDimY = cfg.blockDimZ = 1;
-    cfg.sharedMemBytes = smem;
+    cfg.sharedMemBytes = (unsigned)(2560 + a.stages * stage_bytes + a.raw_ring * 8 * QM_Q4K_ITEM_BYTES);
     cfg.hStream = c->stream;
-    const int kern = ks == 2 ? (r256 ? QM_K_GEMM_Q4K_R256_K128 : QM_K_GEMM_Q4K_K128) : (r256 ? QM_K_GEMM_Q4K_R256 : QM_K_GEMM_Q4K);
-    CUlaunchAttribute coop;
-    if (splitk > 1) {   // the CTAs of a tile wait for one another before they add the shares: all must be resident
-        coop.id = CU_LAUNCH_ATTRIBUTE_COOPERATIVE;
-        coop.value.cooperative = 1;
-        cfg.attrs = &coop;
-        cfg.numAttrs = 1;
-    }
-    DRV(c->drv->cuLaunchKernelEx(&cfg, c->fn[kern], params, nullptr));
+    CUlaunchAttribute attr;
+    attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+    attr.value.clusterDim.x = (unsigned)(p.cg * p.splitk);
+    attr.value.clusterDim.y = attr.value.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    DRV(c->drv->cuLaunchKernelEx(&cfg, c->fn[p.cg == 2 ? QM_K_GEMM_PAIR : QM_K_GEMM_SOLO], params, nullptr));
     c->launches++;
     return QM_OK;
+}
+
+// ---- gate|up matmul of a grouped launch that gathers its rows itself ------------------------------------
+// The activations are the tokens' own matrix a_dev [rows_total][lda]; grouped row p is its row list[p] / topk, and the
+// loader fetches four rows per tile::gather4 copy. One CTA per 256-row tile (128 gate rows, their up rows) and token tile.
+static int32_t gather_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
+                             const QmGemmGroup &g) {
+    if (!g.swiglu || g.experts < 1 || g.gather_topk < 1) return QM_ERR_SHAPE;
+    QmGemmArgs a;
+    memset(&a, 0, sizeof a);
+    const int mt = g.m_typical > 0 ? g.m_typical : m;
+    // (192: lists that fit get a smaller activation tile and with it a fourth stage)
+    const int bn = mt <= 64 ? 64 : mt <= 128 ? 128 : mt <= 192 ? 192 : 256;
+    // Two 64-column chunks per stage where at least two such stages fit: the handshake of a stage costs ~0.3 us, more
+    // than the MMAs of one small chunk.
+    const int chunk_bytes = 2 * 128 * 64 * 2 + bn * 64 * 2;
+    const int ks = (QM_GEMV_SMEM_MAX - 3072) / (2 * chunk_bytes) >= 2 ? 2 : 1;
+    const int stage_bytes = ks * chunk_bytes;
+    const int stages = std::max(2, std::min(8, (QM_GEMV_SMEM_MAX - 3072) / stage_bytes));
+    const cuuint64_t dims[2] = {(cuuint64_t)w->cols, (cuuint64_t)rows_total};
+    const cuuint64_t strides[1] = {(cuuint64_t)lda * 2};
+    const cuuint32_t row_box[2] = {64, 1};   // tile::gather4 names the four rows itself
+    const cuuint32_t estr[2] = {1, 1};
+    DRV(c->drv->cuTensorMapEncodeTiled(&a.tmap_gather, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)(uintptr_t)a_dev,
+                                       dims, strides, row_box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+    const int64_t gate_rows = w->rows / 2;
+    a.status = (unsigned int *)(uintptr_t)c->status_dev;
+    a.n = (int32_t)gate_rows;
+    a.units = w->units;
+    a.tiles16 = (int32_t)((w->rows + 15) / 16);
+    a.bn = bn;
+    a.stages = stages;
+    a.wq_list = (const uint8_t *const *)(uintptr_t)g.wq_list_dev;
+    a.offsets = (const int32_t *)(uintptr_t)g.offsets_dev;
+    a.up_offset = (int32_t)gate_rows;
+    a.h = (uint16_t *)(uintptr_t)g.h_dev;
+    a.ldh = g.ldh;
+    a.gather_list = (const int32_t *)(uintptr_t)g.gather_list_dev;
+    a.gather_topk = g.gather_topk;
+#ifdef QM_DEBUG
+    a.debug = env_int("QM_GEMM_DEBUG", 0);
+#endif
+    void *params[1] = {&a};
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDimX = (unsigned)((gate_rows + 127) / 128);
+    cfg.gridDimY = (unsigned)g.experts;
+    cfg.gridDimZ = (unsigned)((m + bn - 1) / bn);
+    cfg.blockDimX = 576;   // loader warp, MMA warp, sixteen dequantizing warps
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    // alignment slack, stages, barriers, the loader warp's table of token numbers
+    cfg.sharedMemBytes = (unsigned)(1024 + stages * stage_bytes + 512 + 1024);
+    cfg.hStream = c->stream;
+    DRV(c->drv->cuLaunchKernelEx(&cfg, c->fn[ks == 2 ? QM_K_GEMM_GATHER_K128 : QM_K_GEMM_GATHER], params, nullptr));
+    c->launches++;
+    return QM_OK;
+}
+
+// ---- prefill matmul (tcgen05) ----------------------------------------------------------------
+// Single matrix: g.experts == 0, weights w, activations a_dev [m][lda]. Grouped over experts (g.experts > 0): expert
+// e's activation rows are [offsets[e], offsets[e+1]) of a_dev [rows_total][lda], its weights wq_list[e] (all experts
+// shaped like w); m bounds the lists. With g.swiglu the weights are gate|up matrices [2*ffn][k] and the launch stores
+// bf16 silu(gate)*up to g.h instead of C.
+int32_t qm_gemm_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
+                       uint64_t c_dev, int64_t ldc, const QmGemmGroup &g) {
+    if (g.gather_list_dev) return gather_launch(c, w, a_dev, m, rows_total, lda, g);
+    return pair_launch(c, w, a_dev, m, rows_total, lda, c_dev, ldc, g);
 }
 
 extern "C" int32_t qm_matmul_bf16(qm_ctx *c, qm_weight h, uint64_t a_dev, int32_t m, int64_t lda, uint64_t c_dev,

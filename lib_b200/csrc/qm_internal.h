@@ -9,7 +9,7 @@
 #define QM_CTX_MAGIC 0x514D4358u     // "QMCX"
 #define QM_WEIGHT_MAGIC 0x514D5754u  // "QMWT"
 
-enum { QM_MOD_GEMV = 0, QM_MOD_DEQUANT, QM_MOD_Q4K, QM_MOD_GEMM, QM_MOD_MOE, QM_MOD_KQ, QM_MOD_Q81, QM_MOD_COUNT };
+enum { QM_MOD_GEMV = 0, QM_MOD_DEQUANT, QM_MOD_Q4K, QM_MOD_GEMM, QM_MOD_PAIR, QM_MOD_MOE, QM_MOD_KQ, QM_MOD_Q81, QM_MOD_COUNT };
 enum {
     QM_K_GEMV_Q40_M4 = 0, QM_K_GEMV_Q40_M8, QM_K_GEMV_Q80_M4,
     QM_K_GEMV_Q80_M8, QM_K_DEQUANT_Q4K, QM_K_DEQUANT_Q2K, QM_K_DEQUANT_Q40, QM_K_DEQUANT_Q80,
@@ -18,7 +18,7 @@ enum {
     QM_K_FUSED_Q4K_DD_C4D2_TP, QM_K_FUSED_Q4K_DD_C4D3_TP, QM_K_FUSED_Q4K_DD_C4D4_TP,
     QM_K_FUSED_Q4K_DD_C2D2_TP, QM_K_FUSED_Q4K_DD_C2D3_TP, QM_K_FUSED_Q4K_DD_C2D4_TP,
     QM_K_SUM_PARTS, QM_K_REPACK_PARTS,
-    QM_K_GEMM_Q4K, QM_K_GEMM_Q4K_R256, QM_K_GEMM_Q4K_K128, QM_K_GEMM_Q4K_R256_K128, QM_K_MOE_ROUTE, QM_K_MOE_LISTS, QM_K_MOE_GATHER, QM_K_MOE_COMBINE,
+    QM_K_GEMM_GATHER, QM_K_GEMM_GATHER_K128, QM_K_GEMM_PAIR, QM_K_GEMM_SOLO, QM_K_MOE_ROUTE, QM_K_MOE_LISTS, QM_K_MOE_GATHER, QM_K_MOE_COMBINE,
     QM_K_DEQUANT_IQ2XXS, QM_K_GEMV_Q2K_M1, QM_K_GEMV_Q2K_M2, QM_K_GEMV_Q2K_M4, QM_K_GEMV_Q2K_M8,
     QM_K_GEMV_IQ2XXS_M1, QM_K_GEMV_IQ2XXS_M2, QM_K_GEMV_IQ2XXS_M4, QM_K_GEMV_IQ2XXS_M8,
     QM_K_GEMV_Q2K_Q81_M1, QM_K_GEMV_Q2K_Q81_M2, QM_K_GEMV_Q2K_Q81_M4, QM_K_GEMV_Q2K_Q81_M8,
@@ -46,6 +46,7 @@ struct qm_ctx {
     bool have_ctx;
     int sm_count, l2_bytes;
     CUmodule modules[QM_MOD_COUNT];
+    int gemm_clusters[2][5];   // [CTAs per tile - 1][K shares]: clusters of the matmul by CTA pairs that run at once
     CUfunction fn[QM_K_COUNT];
     CUstream own_stream, stream;
     CUdeviceptr status_dev, tickets_dev, partials_dev, gridbar_dev;
@@ -101,7 +102,9 @@ QmWeight *qm_weight_from_handle(qm_weight h);
 int32_t qm_launch(qm_ctx *c, int kernel, unsigned gx, unsigned gy, unsigned block, unsigned smem, void *args,
                   bool pdl);
 int32_t qm_launch_ex(qm_ctx *c, int kernel, unsigned gx, unsigned block, unsigned smem, void *args, bool pdl,
-                     bool cooperative);
+                     bool cooperative, int cluster = 1);
+// Clusters of `cluster` CTAs of this kernel that the device runs at once (0: none).
+int qm_max_clusters(qm_ctx *c, int kernel, int cluster, unsigned block, unsigned smem);
 // Integer tensor-core path for Q4_K: plan for activation rows m and the largest K (in units)
 // of the ops; QM_ERR_SHAPE when the activation planes do not fit in shared memory.
 int qm_fused_grid(qm_ctx *c);

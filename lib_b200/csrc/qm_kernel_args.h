@@ -164,44 +164,50 @@ struct QmFusedArgs {
 
 // Prefill GEMM over Q4_K weights (tcgen05): C[m][n] = sum_k A[m][k] * W[n][k].
 struct QmGemmArgs {
-    alignas(64) CUtensorMap tmap_act;  // activations [m][k] bf16, box 64 x bn, 128-byte swizzle
+    const uint8_t *const *wq_list;   // device array of the experts' gate|up stores (tiled Q4_K)
+    const int32_t *offsets;          // device array [experts + 1]: expert e's rows are [offsets[e], offsets[e+1])
+    const int32_t *gather_list;      // grouped row p is row gather_list[p] / gather_topk of the tokens' own matrix
+    unsigned int *status;
+    uint16_t *h;           // bf16 silu(gate) * up [rows][ldh]
+    int64_t ldh;
+    int32_t n;             // gate rows
+    int32_t up_offset;     // the up rows lie up_offset below the gate rows
+    int32_t units;         // K / 256
+    int32_t tiles16;       // 16-row tiles of a store
+    int32_t bn;            // tokens per CTA: 64, 128, 192 or 256
+    int32_t stages;        // shared-memory stages, 2..8
+    int32_t gather_topk;
+    int32_t debug;         // 0 in production; bits switch off pipeline roles for timing experiments (results are wrong)
+    alignas(64) CUtensorMap tmap_gather;   // the tokens' matrix, box 64 columns x 1 row, 128-byte swizzle
+};
+
+// Matmul by CTA pairs (qm_gemm_pair.cu): 256 weight rows x bn tokens per tile, dequantized weights in tensor memory.
+struct QmPairArgs {
+    alignas(64) CUtensorMap tmap_act;  // activations [tokens][k] bf16, box 64 x box_rows, 128-byte swizzle
     const uint8_t *wq;     // tiled Q4_K store
     float *c;              // [m][ldc]
     unsigned int *status;
     int64_t ldc;
-    int32_t m, n;
+    int32_t m, n;          // tokens and output columns
     int32_t units;         // K / 256
     int32_t tiles16;       // 16-row tiles of the store
-    int32_t bn;            // tokens per CTA: 64, 128, 256 or 512
-    int32_t stages;        // shared-memory stages, 2..8
-    int32_t splitk;        // K shares (blockIdx.z) of a single matmul; 1 in grouped launches
-    // Grouped launch over the experts of a mixture-of-experts layer (blockIdx.z = expert): the
-    // activations are the rows [offsets[e], offsets[e+1]) of one gathered matrix, the weights
-    // of expert e start at wq_list[e]; CTAs beyond an expert's rows leave at once.
-    int32_t grouped;
+    int32_t bn;            // tokens per tile, a multiple of 32 up to 256
+    int32_t nacc;          // accumulators in tensor memory: 2 where they leave room for four stages (bn <= 128), else 1
+    int32_t stages;        // 128-column stages (A in tensor memory, B in shared memory), 4..8: nacc * bn + 64 * stages <= 512
+    int32_t raw_ring;      // units of weight items in shared memory, 4 to 8
+    int32_t box_rows;      // token rows per tile load; a CTA's share of bn is a multiple of it
+    int32_t row_tiles;     // tiles of 128 rows per CTA (SwiGLU: 64 gate rows and their up rows)
+    int32_t items;         // single matmul: tiles (row tile fastest)
+    int32_t splitk;        // pairs of a cluster that share a tile's K range: 1, 2 or 4; above 1 one tile per cluster
+    // Grouped launch: tokens are the rows [offsets[e], offsets[e+1]) of one matrix, the weights of expert e start at
+    // wq_list[e]; an expert without rows has no tiles.
+    int32_t grouped, experts;
     const uint8_t *const *wq_list;   // device array of the experts' stores
     const int32_t *offsets;          // device array [experts + 1]
-    // SwiGLU epilogue (256-row kernel only): sub-tile 0 holds gate rows n, sub-tile 1 the up rows
-    // n + up_offset; the CTA stores bf16 silu(gate) * up to h[row][n] instead of C.
+    // SwiGLU epilogue: n = gate rows, the up rows lie up_offset below; bf16 silu(gate) * up goes to h[row][n].
     int32_t swiglu, up_offset;
     uint16_t *h;           // bf16 [rows][ldh]
     int64_t ldh;
-    int32_t debug;         // 0 in production; bits switch off pipeline roles for timing experiments (results are wrong)
-    int32_t groups;        // groups of dequantizing warps, each a chunk ahead of the next: 4 (one thread per weight row) or 2
-    // Split K: share z of an output tile goes to partials[z][m][n] (plain stores); when all splitk CTAs of
-    // the tile have arrived (tickets[2*tile], zero between launches) each adds one band of the tile in order
-    // of z and writes C — no atomics on C, the same bits every run. The launch is cooperative.
-    float *partials;
-    unsigned int *tickets;
-    int64_t wait_cycles;
-    // Gather folded into the activation load (grouped launches): row p of the grouped order is row
-    // gather_list[p] / gather_topk of the tokens' own matrix, which tmap_gather describes with a box of
-    // 64 columns x 1 row; the loader warp fetches four rows per tile::gather4 copy.
-    const int32_t *gather_list;   // null: the activations are already grouped (tmap_act, tiled loads)
-    int32_t gather_topk;
-    int32_t box_rows;             // token rows per tiled load of tmap_act
-    int32_t plane_rows;           // activation rows of one split-K plane (m, or all grouped rows)
-    alignas(64) CUtensorMap tmap_gather;
 };
 
 #define QM_MAX_EXPERTS 256    // experts of a layer (router, dispatch lists, grouped matmuls); 64 per GPU in expert-parallel runs

@@ -2,6 +2,7 @@
 // matmul that reuses the quantized prefill GEMM over per-expert token lists.
 // The Go-facing surface it stands behind is lm/moe: GroupedTopKRouter.Route
 // (lm/moe/moe.go:73-141) for the routing; the grouped matmul is new API of this path.
+#include <math.h>
 #include <string.h>
 
 #include <algorithm>
@@ -268,11 +269,10 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
     }
     const CUdeviceptr ws = c->moe_ws3;
     if (ffn & 127) return QM_ERR_SHAPE;
-    // Default: the list lengths are read back once, so that the grouped launches have exactly the
-    // token tiles that hold rows (measured 0.75 ms per Mixtral-shaped layer). QM_MOE_NOSYNC=1
-    // keeps everything on the device instead: the launches then cover the longest possible list
-    // (all pairs) and the CTAs beyond an expert's rows leave at once — no synchronization, but
-    // those thousands of empty CTAs each hold an SM's shared memory for a moment (0.95 ms).
+    // Default: the list lengths stay on the device. The matmul's pairs of CTAs walk the lists themselves, so the launch
+    // needs no lengths, only a token tile (chosen for the mean list plus two standard deviations of a random choice):
+    // 435 us per Mixtral-shaped layer of 512 tokens. QM_MOE_NOSYNC=0 reads them back and chooses the tile for the
+    // longest list: 455 us, the difference being the wait.
     // QM_MOE_FOLD=1: the gate|up matmul fetches each grouped row from the token's own row of x (its
     // loader warp follows the dispatch list with tile::gather4 copies), so no gathered copy is written.
     // Same bits as the separate gather pass (the matmul sees the same rows in the same order), but
@@ -281,7 +281,8 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
     // 0.82 ms; the same loader with 16-byte cp.async from one warp: 1.32 ms), while the pass it
     // saves costs about 5 us. So the separate pass stays the default.
     const bool fold = qm_env_int("QM_MOE_FOLD", 0) != 0 && (x_bf16_dev & 15) == 0 && (ldx & 7) == 0;
-    const bool nosync = qm_env_int("QM_MOE_NOSYNC", 0) != 0;
+    // (that launch still has one CTA per row tile and token tile, so it reads the lengths back unless told otherwise)
+    const bool nosync = qm_env_int("QM_MOE_NOSYNC", fold ? 0 : 1) != 0;
     if (fold) {
         int32_t counts[QM_MAX_EXPERTS];
         CUdeviceptr offsets_dev = 0, list_dev = 0;
@@ -319,7 +320,9 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
     {
         CtxGuard g(c);
         DRV(g.rc);
-        const int32_t typical = (int32_t)std::max<int64_t>(1, (pairs + experts - 1) / experts);
+        if (pairs >= (1 << 24)) return QM_ERR_SHAPE;   // as qm_moe_experts
+        const double mean = (double)pairs / experts;
+        const int32_t typical = (int32_t)std::max(1.0, mean + 2.0 * sqrt(mean));
         rc = experts_launch(c, wg, wd, experts, ws + o_rows, pairs, (int32_t)pairs, typical, offsets_dev, ws + o_y, hidden,
                             ffn);
         if (rc) return rc;
