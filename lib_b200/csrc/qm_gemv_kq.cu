@@ -342,13 +342,166 @@ __device__ __forceinline__ void gemv_kq_body(const QmKqArgs &a) {
     }
 }
 
+// ---- one Q8_1 row, K up to 4096: activations in registers ---------------------------------------
+// A lane always meets the same Q8_1 blocks (block lane & 7 of the super-blocks lane >> 3, + 4, ...), so they are
+// read from shared memory once and stay in registers over the warp's rows: STEPS blocks of eight words and a
+// factor (Q2_K: and the two group sums that meet the minima). What a row then costs per step is its codes.
+//
+// IQ2_XXS. A codebook byte is one of 8, 25, 43 (its high nibble is 0, 1, 2), so an entry is held as eight PRMT
+// selector nibbles; the signs of an entry are the third bits of the same nibbles, looked up by the seven sign bits.
+// One OR joins them and two PRMTs over {8, 25, 43, -8, -25, -43} give the eight signed bytes: 11 instructions per
+// entry instead of about 27 (64-bit codebook, parity, mask multiply, separate dot product of the negated bytes).
+// Both tables are held kCopies times, interleaved, so that the lanes' random reads meet few bank conflicts.
+constexpr int kCopies = 8;
+
+template <int FMT, int STEPS>
+__device__ __forceinline__ void gemv_kq_q81_row1(const QmKqArgs &a, uint32_t *tab) {   // tab: 256 codebook entries, 128 sign patterns
+    constexpr int kBlockBytes = FMT == 10 ? 84 : 66;
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int slot = blockIdx.y;
+    const uint8_t *wq = a.wq;
+    float *y = a.y + (int64_t)slot * a.y_slot_stride;
+    const uint8_t *x = static_cast<const uint8_t *>(a.x) + (int64_t)slot * a.x_slot_stride * 36;
+    const int64_t row_bytes = (int64_t)a.units * kBlockBytes;
+    extern __shared__ __align__(16) uint8_t dyn_smem[];
+    if (a.ids) {
+        const int e = a.ids[slot];
+        if (e < 0 || e >= a.experts) {
+            for (int64_t row = wid * 32 + lane; row < a.rows; row += (int64_t)warps * 32) y[row] = __int_as_float(0x7fffffff);
+            return;
+        }
+        wq += (int64_t)e * a.rows * row_bytes;
+    }
+    // ring of rows, as in gemv_kq_body
+    const int D = a.depth;
+    uint8_t *ring = dyn_smem + a.xs_bytes + (threadIdx.x >> 5) * D * (uint32_t)row_bytes;
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+    const int pieces = (int)(row_bytes >> 4);
+    int64_t p_row = wid;
+    int p_slot = 0;
+    auto issue = [&]() {
+        if (p_row < a.rows) {
+            const uint8_t *src = wq + p_row * row_bytes;
+            const uint32_t dst = ring_s + (uint32_t)p_slot * (uint32_t)row_bytes;
+            for (int i = lane; i < pieces; i += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 16 * i) : "memory");
+            p_row += warps;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        p_slot = p_slot + 1 == D ? 0 : p_slot + 1;
+    };
+    for (int d = 0; d < D; d++) issue();
+    for (int i = threadIdx.x; i < a.units * 72; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(dyn_smem)[i] = __ldg(reinterpret_cast<const uint32_t *>(x) + i);
+    if (FMT == 16) {
+        for (int i = threadIdx.x; i < 384; i += blockDim.x) {
+            uint32_t w = 0;
+            if (i < 256) {
+                const unsigned long long code = QM_IQ2XXS_GRID_INIT[i];
+#pragma unroll
+                for (int k = 0; k < 8; k++) w |= (uint32_t)((code >> (8 * k + 4)) & 3ull) << (4 * k);
+            } else {
+                const uint32_t si = i - 256, signs = si | ((uint32_t)(__popc(si) & 1) << 7);
+#pragma unroll
+                for (int k = 0; k < 8; k++) w |= ((signs >> k) & 1u) << (4 * k + 2);
+            }
+#pragma unroll
+            for (int k = 0; k < kCopies; k++) tab[i * kCopies + k] = w;
+        }
+    }
+    __syncthreads();
+    const int i8 = lane & 7;   // the lane's Q8_1 block within its super-blocks
+    int xw[STEPS][8];
+    float dx[STEPS], xs0[FMT == 10 ? STEPS : 1], xs1[FMT == 10 ? STEPS : 1];
+#pragma unroll
+    for (int s = 0; s < STEPS; s++) {
+        const int u = min((lane >> 3) + 4 * s, a.units - 1);
+        const uint32_t *xb = reinterpret_cast<const uint32_t *>(dyn_smem) + (u * 8 + i8) * 9;
+        dx[s] = h2f(xb[0] & 0xFFFFu);
+#pragma unroll
+        for (int w = 0; w < 8; w++) xw[s][w] = (int)xb[1 + w];
+        if (FMT == 10) {
+            int s0 = 0, s1 = 0;
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                s0 = __dp4a(0x01010101, xw[s][w], s0);
+                s1 = __dp4a(0x01010101, xw[s][4 + w], s1);
+            }
+            xs0[s] = small_int_to_float(s0);
+            xs1[s] = small_int_to_float(s1);
+        }
+    }
+    int c_slot = 0;
+    for (int64_t row = wid; row < a.rows; row += warps) {
+        if (D == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else if (D == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 3;" ::: "memory");
+        __syncwarp();
+        const uint8_t *wr = ring + (size_t)c_slot * (size_t)row_bytes;
+        float acc = 0.f;
+#pragma unroll
+        for (int s = 0; s < STEPS; s++) {
+            const int u = (lane >> 3) + 4 * s;
+            if (u >= a.units) continue;
+            const uint8_t *blk = wr + u * kBlockBytes;
+            if (FMT == 10) {
+                // elements 32 i8 .. +31: the 32 bytes of half i8>>2, bit pair i8&3; scale groups 2 i8 and 2 i8 + 1
+                const int sh = 2 * (i8 & 3);
+                const uint32_t *qw = reinterpret_cast<const uint32_t *>(blk + 16 + 32 * (i8 >> 2));
+                const uint32_t sc2 = *reinterpret_cast<const uint16_t *>(blk + 2 * i8);
+                const uint32_t dd = *reinterpret_cast<const uint32_t *>(blk + 80);
+                const float d = h2f(dd & 0xFFFFu), dmin = h2f(dd >> 16);
+                const float dsc0 = d * (float)(sc2 & 0x0Fu), dmn0 = dmin * (float)((sc2 >> 4) & 0x0Fu);
+                const float dsc1 = d * (float)((sc2 >> 8) & 0x0Fu), dmn1 = dmin * (float)(sc2 >> 12);
+                int dot0 = 0, dot1 = 0;
+#pragma unroll
+                for (int w = 0; w < 4; w++) {
+                    dot0 = __dp4a((int)((qw[w] >> sh) & 0x03030303u), xw[s][w], dot0);
+                    dot1 = __dp4a((int)((qw[4 + w] >> sh) & 0x03030303u), xw[s][4 + w], dot1);
+                }
+                const float g0 = dsc0 * small_int_to_float(dot0) - dmn0 * xs0[s];   // |.| <= 16*3*127
+                const float g1 = dsc1 * small_int_to_float(dot1) - dmn1 * xs1[s];
+                acc = fmaf(dx[s], g0 + g1, acc);
+            } else {
+                const float d = h2f(*reinterpret_cast<const uint16_t *>(blk));
+                const uint16_t *g16 = reinterpret_cast<const uint16_t *>(blk + 2 + 8 * i8);
+                const uint32_t indices = (uint32_t)g16[0] | ((uint32_t)g16[1] << 16);
+                const uint32_t aux = (uint32_t)g16[2] | ((uint32_t)g16[3] << 16);
+                const float scale = (0.125f * d) * (float)(2u * (aux >> 28) + 1u);
+                int all = 0;
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    const uint32_t sel = tab[((indices >> (8 * l)) & 0xFFu) * kCopies + i8] |
+                                         tab[(256u + ((aux >> (7 * l)) & 127u)) * kCopies + i8];
+                    // (bit 3 of a selector nibble is clear; PRMT reads the low four nibbles)
+                    all = __dp4a((int)__byte_perm(0x002B1908u, 0x00D5E7F8u, sel), xw[s][2 * l], all);
+                    all = __dp4a((int)__byte_perm(0x002B1908u, 0x00D5E7F8u, sel >> 16), xw[s][2 * l + 1], all);
+                }
+                acc = fmaf(scale * dx[s], small_int_to_float(all), acc);   // |.| <= 32*43*127
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) y[row] = acc;
+        __syncwarp();   // every lane has read the slot before the next copy overwrites it
+        issue();
+        c_slot = c_slot + 1 == D ? 0 : c_slot + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 }  // namespace
 
 // Instantiated for 1, 2, 4 and 8 activation rows (the host picks the smallest that holds m), each for float32
 // and for Q8_1 activations.
 #define QM_KQ_KERNEL(name, fmt, mm, xq)                                                                        \
     extern "C" __global__ void __launch_bounds__(256) name(const __grid_constant__ QmKqArgs a) {               \
-        if (a.depth >= 2) gemv_kq_body<fmt, mm, xq, true>(a);                                                  \
+        __shared__ uint32_t tab[xq && mm == 1 && fmt == 16 ? 384 * kCopies : 1];                               \
+        if (xq && mm == 1 && a.depth >= 2 && a.units <= 8) gemv_kq_q81_row1<fmt, 2>(a, tab);                   \
+        else if (xq && mm == 1 && a.depth >= 2 && a.units <= 16) gemv_kq_q81_row1<fmt, 4>(a, tab);             \
+        else if (a.depth >= 2) gemv_kq_body<fmt, mm, xq, true>(a);                                             \
         else gemv_kq_body<fmt, mm, xq, false>(a);                                                              \
     }
 QM_KQ_KERNEL(qm_gemv_q2k_m1, 10, 1, false)
