@@ -135,7 +135,26 @@ struct Cursor {   // walks the items of this warp, op after op
 // NAT: the weights keep the order of the GGUF block (mma k index i <-> element i of the sub-block), as
 // the Q4_0 / Q8_0 stores do; otherwise k index 4t+i <-> element 8t+i, 16+4t+i <-> element 8t+4+i, the
 // order of the tiled Q4_K store.
-template <int NT, bool NAT = false>
+// CS > 1: the CTAs of a cluster share the quantization of x, and what one of them has quantized goes into the
+// shared memory of all CS of them (xs_b, xsum_b, sxw_b lie at the same place in each).
+template <int CS, typename T>
+__device__ __forceinline__ T *in_cta(T *p, int rank) {   // the place of p in CTA `rank` of the cluster
+    if (CS == 1) return p;
+    T *d;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(d) : "l"(p), "r"(rank));
+    return d;
+}
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+template <int CS>
+__device__ __forceinline__ void cta_barrier() {   // over the CTA, or over the cluster that shares a staging
+    if (CS == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <int NT, bool NAT = false, int CS = 1>
 __device__ __forceinline__ float quantize_pair(const float (&v)[8], int j, int ul, int lane, int NL, int CPM,
                                                uint8_t *xs_b, int pstride, uint32_t *xsum_b, float *sxw_b,
                                                float wmul = 1.f) {
@@ -174,33 +193,37 @@ __device__ __forceinline__ float quantize_pair(const float (&v)[8], int j, int u
     // lane = 4*sub-block + t': this lane's 8 columns are the B fragment of lane t' for
     // sub-block sb; the fragments of sub-blocks 2p and 2p+1 sit side by side
     const int sb = lane >> 2, tq = lane & 3;
-    if (NAT) {
-        // elements 8tq..8tq+3 are register b[tq >> 1] of lane t' = 2*(tq & 1), the next four that of lane t' + 1
-        const int off = ((ul * 4 + (sb >> 1)) * 4 + 2 * (tq & 1)) * 16 + (sb & 1) * 8 + (tq >> 1) * 4;
-        for (int l = 0; l < NL; l++) {
-            uint8_t *pl = xs_b + (size_t)(j * NL + l) * pstride + off;
-            *reinterpret_cast<uint32_t *>(pl) = w0[l];
-            *reinterpret_cast<uint32_t *>(pl + 16) = w1[l];
-        }
-    } else {
-        const int off = ((ul * 4 + (sb >> 1)) * 4 + tq) * 16 + (sb & 1) * 8;
-        for (int l = 0; l < NL; l++)
-            *reinterpret_cast<uint2 *>(xs_b + (size_t)(j * NL + l) * pstride + off) = make_uint2(w0[l], w1[l]);
-    }
     const int n0 = j * CPM;   // first mma column of this activation row
-    if (tq == 0) {
-        // sub-block sums in units of the unit's maximum (|.| <= 32): safe in fp16 whatever
-        // the magnitude of the activations; the factor comes back with the column weight
-        const float sn = sum * inv * (1.f / 127.f);
-        const __half sh = __float2half_rn(sn);
-        const __half sl = __float2half_rn(sn - __half2float(sh));
-        __half *xh = reinterpret_cast<__half *>(xsum_b);
-        xh[((size_t)ul * 8 * NT + n0) * 8 + sb] = sh;
-        xh[((size_t)ul * 8 * NT + n0 + 1) * 8 + sb] = sl;
-    }
-    if (lane < CPM) {
-        const float lw = lane == 0 ? 1.f : lane == 1 ? (1.f / 128.f) : lane == 2 && NL == 3 ? (1.f / 16384.f) : 0.f;
-        sxw_b[(size_t)ul * 8 * NT + n0 + lane] = sx * lw * wmul;   // wmul: a constant the consumer folds into the column weight
+#pragma unroll
+    for (int c = 0; c < CS; c++) {
+        uint8_t *xs_c = in_cta<CS>(xs_b, c);
+        if (NAT) {
+            // elements 8tq..8tq+3 are register b[tq >> 1] of lane t' = 2*(tq & 1), the next four that of lane t' + 1
+            const int off = ((ul * 4 + (sb >> 1)) * 4 + 2 * (tq & 1)) * 16 + (sb & 1) * 8 + (tq >> 1) * 4;
+            for (int l = 0; l < NL; l++) {
+                uint8_t *pl = xs_c + (size_t)(j * NL + l) * pstride + off;
+                *reinterpret_cast<uint32_t *>(pl) = w0[l];
+                *reinterpret_cast<uint32_t *>(pl + 16) = w1[l];
+            }
+        } else {
+            const int off = ((ul * 4 + (sb >> 1)) * 4 + tq) * 16 + (sb & 1) * 8;
+            for (int l = 0; l < NL; l++)
+                *reinterpret_cast<uint2 *>(xs_c + (size_t)(j * NL + l) * pstride + off) = make_uint2(w0[l], w1[l]);
+        }
+        if (tq == 0) {
+            // sub-block sums in units of the unit's maximum (|.| <= 32): safe in fp16 whatever
+            // the magnitude of the activations; the factor comes back with the column weight
+            const float sn = sum * inv * (1.f / 127.f);
+            const __half sh = __float2half_rn(sn);
+            const __half sl = __float2half_rn(sn - __half2float(sh));
+            __half *xh = reinterpret_cast<__half *>(in_cta<CS>(xsum_b, c));
+            xh[((size_t)ul * 8 * NT + n0) * 8 + sb] = sh;
+            xh[((size_t)ul * 8 * NT + n0 + 1) * 8 + sb] = sl;
+        }
+        if (lane < CPM) {
+            const float lw = lane == 0 ? 1.f : lane == 1 ? (1.f / 128.f) : lane == 2 && NL == 3 ? (1.f / 16384.f) : 0.f;
+            in_cta<CS>(sxw_b, c)[(size_t)ul * 8 * NT + n0 + lane] = sx * lw * wmul;   // wmul: a constant the consumer folds into the column weight
+        }
     }
     return sq;
 }
@@ -945,12 +968,13 @@ __device__ __forceinline__ void cp_async_wait_n() {
 // adds the partial vectors of a producer that ran in K parts, applies the input transform and
 // quantizes into limb planes, sub-block sums and column weights; leaves each warp's part of the
 // sums of squares in ssq. Returns the thread's "gave up waiting" flag.
-template <int CPM, bool TP, int NT = 1>
+template <int CPM, bool TP, int NT = 1, int CS = 1>
 __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, uint8_t *xs, int plane_stride,
                                       uint32_t *xsum, float *sxw, float *ssq, bool dead) {
     const QmFusedArgs &a = *ap;
-    constexpr int C = 16, NL = CPM == 4 ? 3 : 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // W warps share the staging: this CTA's sixteen, or those of all CS CTAs of the cluster
+    constexpr int W = 16 * CS, NL = CPM == 4 ? 3 : 2;
+    const int lane = threadIdx.x & 31, warp = (CS == 1 ? 0 : cluster_rank() * 16) + (threadIdx.x >> 5);
     const int M = a.m;
     const int nun = po->units, xop = po->xop;
     const float *opx = po->x, *opx2 = po->x2;
@@ -964,7 +988,11 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
             const bool poll = po->barrier != 0;   // x is an earlier op's output
             float sq_run = 0.f;
             int sq_j = -1;
-            if (norm && lane < 8) ssq[lane * 16 + warp] = 0.f;
+            auto put_ssq = [&](int j, float v) {   // this warp's share of row j's sum of squares, to every CTA
+#pragma unroll
+                for (int k = 0; k < CS; k++) in_cta<CS>(ssq, k)[j * W + warp] = v;
+            };
+            if (norm && lane < 8) put_ssq(lane, 0.f);
             __syncwarp();
             auto load_x = [&](int idx, float4 (&r)[4]) {
                 const int j = idx / nun, ul = idx - j * nun;
@@ -980,7 +1008,7 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
             // x given as several partial vectors (the producer was cut into K parts): all of them are
             // in flight at once, one (row, unit) pair per warp and round
             if (x_parts > 1) {
-                for (int idx = warp; idx < total; idx += C) {
+                for (int idx = warp; idx < total; idx += W) {
                     const int j = idx / nun, ul = idx - j * nun;
                     const float *xp = opx + (int64_t)j * ldx + col0 + ul * QM_K_UNIT + lane * 8;
                     float4 r[8];
@@ -1037,13 +1065,13 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
                                 v[4] += r[2 * k + 1].x; v[5] += r[2 * k + 1].y; v[6] += r[2 * k + 1].z; v[7] += r[2 * k + 1].w;
                             }
                     }
-                    const float sq = quantize_pair<NT>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 0.0625f);
+                    const float sq = quantize_pair<NT, false, CS>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 0.0625f);
                     if (norm) {
                         if (j != sq_j) {
                             if (sq_j >= 0) {
 #pragma unroll
                                 for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
-                                if (lane == 0) ssq[sq_j * 16 + warp] = sq_run;
+                                if (lane == 0) put_ssq(sq_j, sq_run);
                             }
                             sq_j = j;
                             sq_run = 0.f;
@@ -1077,13 +1105,13 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
                     for (int e = 0; e < 8; e++)
                         v[e] = xop == 2 ? v[e] + w[e] : v[e] / (1.f + __expf(-v[e])) * w[e];
                 }
-                const float sq = quantize_pair<NT>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 0.0625f);
+                const float sq = quantize_pair<NT, false, CS>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 0.0625f);
                 if (norm) {   // per-warp running sum of squares of activation row j
                     if (j != sq_j) {
                         if (sq_j >= 0) {
 #pragma unroll
                             for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
-                            if (lane == 0) ssq[sq_j * 16 + warp] = sq_run;
+                            if (lane == 0) put_ssq(sq_j, sq_run);
                         }
                         sq_j = j;
                         sq_run = 0.f;
@@ -1094,13 +1122,13 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
             {
                 float4 rawA[4], rawB[4];
                 if (warp < total) load_x(warp, rawA);
-                if (warp + C < total) load_x(warp + C, rawB);
-                for (int idx = warp; idx < total; idx += 2 * C) {
+                if (warp + W < total) load_x(warp + W, rawB);
+                for (int idx = warp; idx < total; idx += 2 * W) {
                     consume(idx, rawA);
-                    if (idx + 2 * C < total) load_x(idx + 2 * C, rawA);
-                    if (idx + C < total) {
-                        consume(idx + C, rawB);
-                        if (idx + 3 * C < total) load_x(idx + 3 * C, rawB);
+                    if (idx + 2 * W < total) load_x(idx + 2 * W, rawA);
+                    if (idx + W < total) {
+                        consume(idx + W, rawB);
+                        if (idx + 3 * W < total) load_x(idx + 3 * W, rawB);
                     }
                 }
             }
@@ -1108,7 +1136,7 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
             if (sq_j >= 0) {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
-                if (lane == 0) ssq[sq_j * 16 + warp] = sq_run;
+                if (lane == 0) put_ssq(sq_j, sq_run);
             }
     }
     return dead;
@@ -1121,7 +1149,7 @@ __device__ __forceinline__ bool dd_stage(const QmFusedArgs *ap, const QmOp *po, 
 // is what lets the host refill the other arena half with the "not yet written" pattern.
 // NT = column tiles of eight mma columns: 1, or 2 with CPM = 2 for five to eight activation rows (each weight
 // fragment then feeds two mma, one per tile; the low- and high-nibble sums share one accumulator).
-template <int CPM, int D, bool TP, bool SEL = false, int NT = 1>
+template <int CPM, int D, bool TP, bool SEL = false, int NT = 1, int CS = 1>
 __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
     constexpr int C = 16;                       // warps per CTA
     constexpr int NL = CPM == 4 ? 3 : 2;        // limbs per activation row
@@ -1136,8 +1164,8 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
     uint8_t *xs = smem;                                                            // [P][plane_stride]
     uint32_t *xsum = reinterpret_cast<uint32_t *>(xs + (size_t)P * plane_stride);   // [units][8*NT][4] f16 pairs
     float *sxw = reinterpret_cast<float *>(xsum + (size_t)a.max_units * 8 * NT * 4);   // [units][8*NT] column weights
-    float *ssq = sxw + (size_t)a.max_units * 8 * NT;                                // [8][16]
-    float *slots = ssq + 8 * 16;                                                    // [C][2][M*16]
+    float *ssq = sxw + (size_t)a.max_units * 8 * NT;                                // [8][16 * CS]
+    float *slots = ssq + 8 * 16 * CS;                                                    // [C][2][M*16]
     QmOp *sop = reinterpret_cast<QmOp *>(((uintptr_t)(slots + (size_t)C * 2 * M * 16) + 15) & ~(uintptr_t)15);   // [2], or [nops] inline
     uint8_t *stages = reinterpret_cast<uint8_t *>(((uintptr_t)(sop + (inl ? QM_MAX_INLINE_OPS : 2)) + 127) & ~(uintptr_t)127);
     uint8_t *my_stages = stages + (size_t)warp * D * kStageBytes;
@@ -1168,6 +1196,17 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
         n = wq + (warp < wrem ? 1 : 0);
     };
 
+    // The CTA's place among those of the op. Independent ops of a list of selected experts start their tiles at
+    // different CTAs (cta_rot), so that the CTAs with one tile more change from op to op.
+    auto cta_index = [&](const QmOp *po) -> int {
+        int c = (int)blockIdx.x - po->cta0;
+        if (SEL) {
+            c += po->cta_rot;
+            if (c >= po->nctas) c -= po->nctas;
+        }
+        return c;
+    };
+
     // ---- producer side of the ring: a pointer and a count per op -------------------------------
     // (a warp's items of an op are one contiguous run of the store)
     int p_op = -1, p_n = 0;
@@ -1178,7 +1217,7 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
             const QmOp *po = ops + p_op;
             int tile0, lo, n, wq, wrem;
             const int units = po->units;
-            warp_range(po->q, po->rem, units, (int)blockIdx.x - po->cta0, po->nctas, tile0, lo, n, wq, wrem);
+            warp_range(po->q, po->rem, units, cta_index(po), po->nctas, tile0, lo, n, wq, wrem);
             if (n > 0) {
                 p_n = n;
                 const uint8_t *wq = po->wq;
@@ -1249,13 +1288,14 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
     for (int opi = 0; opi < a.nops; opi++) {
         const QmOp *po = inl ? &sop[opi] : &sop[opi & 1];
         QM_DD_MARK(0);
-        // every warp has finished with the activation planes and the partial sums of the op before
-        __syncthreads();
+        // every warp (of every CTA that writes into these planes) has finished with the activation planes and the
+        // partial sums of the op before
+        cta_barrier<CS>();
         const int nun = po->units;
         const int xop = po->xop;
         const bool norm = xop == 1 || xop == 2;
         const int parts = po->parts, x_parts = po->x_parts;
-        const int cta_in_grp = (int)blockIdx.x - po->cta0;
+        const int cta_in_grp = cta_index(po);
 
         const float *ssq_in = po->ssq_in;
         // The words of a producer that ran in K parts (its sums of squares per part and row): every lane reads
@@ -1274,7 +1314,7 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
         if (want_w0) ssq_w0 = load_word(lane >> 3);
         if (want_w1) ssq_w1 = load_word((lane >> 3) + 4);
         // ---- stage x: poll until written, quantize into limbs --------------------------------------
-        dead = dd_stage<CPM, TP, NT>(&a, po, xs, plane_stride, xsum, sxw, ssq, dead);
+        dead = dd_stage<CPM, TP, NT, CS>(&a, po, xs, plane_stride, xsum, sxw, ssq, dead);
         {   // a word that had not been written yet: wait for it (bounded)
             auto settle = [&](float &w, int k) {
                 long long t0 = 0;
@@ -1290,7 +1330,7 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
             if (want_w0) settle(ssq_w0, lane >> 3);
             if (want_w1) settle(ssq_w1, (lane >> 3) + 4);
         }
-        __syncthreads();
+        cta_barrier<CS>();
         QM_DD_MARK(1);
         if (!inl && warp == C - 1 && opi + 1 < a.nops && lane < (int)(sizeof(QmOp) / 16))
             reinterpret_cast<uint4 *>(&sop[(opi + 1) & 1])[lane] = __ldg(reinterpret_cast<const uint4 *>(ops + opi + 1) + lane);
@@ -1301,7 +1341,9 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
             const float inv_cols = 1.f / (float)po->cols;
             float *ssq_out = po->ssq_out;
             for (int j = 0; j < M; j++) {
-                float sq = ssq[j * 16 + (lane & 15)];   // the warps' parts, added as a fixed tree
+                float sq = ssq[j * 16 * CS + (lane & 15)];   // the warps' parts, added as a fixed tree
+#pragma unroll
+                for (int k = 1; k < CS; k++) sq += ssq[j * 16 * CS + k * 16 + (lane & 15)];
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
                 if (parts > 1) {
@@ -1545,7 +1587,7 @@ __device__ __forceinline__ void dd_body(const QmFusedArgs &a) {
         if (fin_tile >= 0) {
             // partial sums of the warps that worked on the tile before this one, in warp order
             int t0_, lo_, n_, wq, wrem;
-            warp_range(po->q, po->rem, nun, (int)blockIdx.x - po->cta0, po->nctas, t0_, lo_, n_, wq, wrem);
+            warp_range(po->q, po->rem, nun, cta_index(po), po->nctas, t0_, lo_, n_, wq, wrem);
             const unsigned int ts = (unsigned int)(fin_tile * nun), big = (unsigned int)wrem * (unsigned int)(wq + 1);
             const int wf = wq == 0 ? (int)ts : ts < big ? (int)(ts / (unsigned int)(wq + 1))
                                                          : wrem + (int)((ts - big) / (unsigned int)wq);
@@ -1618,7 +1660,7 @@ __device__ __forceinline__ void mma_s8s8(int (&d)[4], uint32_t a0, uint32_t a1, 
 // K parts (a.parts > 1): the CTAs form a.parts groups, group p multiplies K units [p*units, (p+1)*units) of
 // every tile — it stages only that range of x — and leaves its products, without the RMS scale, in partial
 // vector p (a.y + p*a.part_stride) and its sums of squares in a.ssq[p*8 + row]; qm_lean_sum adds them up.
-template <int FMT, int CPM, int D, int NT>
+template <int FMT, int CPM, int D, int NT, int CS = 1>
 __device__ __forceinline__ void lean_body(const QmLeanArgs &a) {
     constexpr int C = 16;
     constexpr int NL = CPM == 4 ? 3 : 2;
@@ -1634,8 +1676,8 @@ __device__ __forceinline__ void lean_body(const QmLeanArgs &a) {
     uint8_t *xs = smem;                                                             // [P][plane_stride]
     uint32_t *xsum = reinterpret_cast<uint32_t *>(xs + (size_t)P * plane_stride);    // [units][8*NT][4] f16 pairs
     float *sxw = reinterpret_cast<float *>(xsum + (size_t)nun * 8 * NT * 4);         // [units][8*NT] column weights
-    float *ssq = sxw + (size_t)nun * 8 * NT;                                         // [8][16]
-    float *slots = ssq + 8 * 16;                                                     // [C][2][M*16]
+    float *ssq = sxw + (size_t)nun * 8 * NT;                                         // [8][16 * CS]
+    float *slots = ssq + 8 * 16 * CS;                                                     // [C][2][M*16]
     uint8_t *stages = reinterpret_cast<uint8_t *>(((uintptr_t)(slots + (size_t)C * 2 * M * 16) + 127) & ~(uintptr_t)127);
     uint8_t *my_stages = stages + (size_t)warp * D * STAGE;
 
@@ -1682,61 +1724,82 @@ __device__ __forceinline__ void lean_body(const QmLeanArgs &a) {
     for (int d = 0; d < D; d++) issue();
 
     // ---- stage x (the launch's input: no polling), quantize into limb planes --------------------------
+    // The warps of the cluster's CTAs take the (row, unit) pairs in turn, two register sets each: while one pair
+    // is quantized the loads of the next are in flight.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    __syncthreads();
+    cta_barrier<CS>();
     const int xop = a.xop;
     const bool norm = xop == 1 || xop == 2;
     {
+        constexpr int W = C * CS;   // warps that share the staging
+        const int w = (CS == 1 ? 0 : cluster_rank() * C) + warp, total = M * nun;
         float sq_run = 0.f;
         int sq_j = -1;
-        if (norm && lane < 8) ssq[lane * 16 + warp] = 0.f;
-        __syncwarp();
-        for (int idx = warp; idx < M * nun; idx += C) {
-            const int j = idx / nun, ul = idx - j * nun;
-            const int col = (unit0 + ul) * QM_K_UNIT + lane * 8;
-            float v[8];
+        auto put_ssq = [&](int j, float v) {   // this warp's share of row j's sum of squares, to every CTA
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = 0.f;
+            for (int k = 0; k < CS; k++) in_cta<CS>(ssq, k)[j * W + w] = v;
+        };
+        if (norm && lane < 8) put_ssq(lane, 0.f);
+        __syncwarp();
+        auto load_x = [&](int idx, float4 (&r)[4]) {
+            const int j = idx / nun, col = (unit0 + idx - j * nun) * QM_K_UNIT + lane * 8;
+            r[0] = r[1] = r[2] = r[3] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (col < a.cols) {   // cols is a multiple of 32: a lane's eight columns are all inside or all outside
                 const float *xp = a.x + (int64_t)j * a.ldx + col;
-                const float4 r0 = *reinterpret_cast<const float4 *>(xp), r1 = *reinterpret_cast<const float4 *>(xp + 4);
-                v[0] = r0.x; v[1] = r0.y; v[2] = r0.z; v[3] = r0.w; v[4] = r1.x; v[5] = r1.y; v[6] = r1.z; v[7] = r1.w;
+                r[0] = *reinterpret_cast<const float4 *>(xp);
+                r[1] = *reinterpret_cast<const float4 *>(xp + 4);
                 if (xop >= 2) {
                     const float *x2p = a.x2 + (int64_t)j * a.ldx + col;
-                    const float4 s0 = *reinterpret_cast<const float4 *>(x2p), s1 = *reinterpret_cast<const float4 *>(x2p + 4);
-                    const float w[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-                    for (int e = 0; e < 8; e++) v[e] = xop == 2 ? v[e] + w[e] : v[e] / (1.f + __expf(-v[e])) * w[e];
+                    r[2] = *reinterpret_cast<const float4 *>(x2p);
+                    r[3] = *reinterpret_cast<const float4 *>(x2p + 4);
                 }
             }
-            const float sq = quantize_pair<NT, true>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 1.f);
+        };
+        auto flush_ssq = [&]() {
+            if (sq_j < 0) return;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
+            if (lane == 0) put_ssq(sq_j, sq_run);
+        };
+        auto consume = [&](int idx, const float4 (&r)[4]) {
+            const int j = idx / nun, ul = idx - j * nun;
+            float v[8] = {r[0].x, r[0].y, r[0].z, r[0].w, r[1].x, r[1].y, r[1].z, r[1].w};
+            if (xop >= 2) {
+                const float u[8] = {r[2].x, r[2].y, r[2].z, r[2].w, r[3].x, r[3].y, r[3].z, r[3].w};
+                // (columns past the end: 0 + 0, and 0 / 2 * 0)
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = xop == 2 ? v[e] + u[e] : v[e] / (1.f + __expf(-v[e])) * u[e];
+            }
+            const float sq = quantize_pair<NT, true, CS>(v, j, ul, lane, NL, CPM, xs, plane_stride, xsum, sxw, 1.f);
             if (norm) {
                 if (j != sq_j) {
-                    if (sq_j >= 0) {
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
-                        if (lane == 0) ssq[sq_j * 16 + warp] = sq_run;
-                    }
+                    flush_ssq();
                     sq_j = j;
                     sq_run = 0.f;
                 }
                 sq_run += sq;
             }
+        };
+        float4 rA[4], rB[4];
+        if (w < total) load_x(w, rA);
+        for (int idx = w; idx < total; idx += 2 * W) {
+            if (idx + W < total) load_x(idx + W, rB);
+            consume(idx, rA);
+            if (idx + 2 * W < total) load_x(idx + 2 * W, rA);
+            if (idx + W < total) consume(idx + W, rB);
         }
-        if (sq_j >= 0) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq_run += __shfl_xor_sync(0xffffffffu, sq_run, o);
-            if (lane == 0) ssq[sq_j * 16 + warp] = sq_run;
-        }
+        flush_ssq();
     }
-    __syncthreads();
+    cta_barrier<CS>();
     float myscale[NT];
 #pragma unroll
     for (int ct = 0; ct < NT; ct++) myscale[ct] = 1.f;
     if (norm) {
         const float inv_cols = 1.f / (float)a.cols;
         for (int j = 0; j < M; j++) {
-            float sq = ssq[j * 16 + (lane & 15)];
+            float sq = ssq[j * 16 * CS + (lane & 15)];
+#pragma unroll
+            for (int k = 1; k < CS; k++) sq += ssq[j * 16 * CS + k * 16 + (lane & 15)];
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
             if (a.parts > 1) {   // a part leaves its products unscaled and publishes its share of the sum of squares
@@ -1935,21 +1998,31 @@ QM_DD_KERNEL(qm_fused_q4k_dd_c2d2_tp, 2, 2, true)
 QM_DD_KERNEL(qm_fused_q4k_dd_c2d3_tp, 2, 3, true)
 QM_DD_KERNEL(qm_fused_q4k_dd_c2d4_tp, 2, 4, true)
 
-// Five to eight activation rows: two column tiles (D = 2 or 3 stages: sixteen limb planes take the room of the fourth).
-#define QM_DD8_KERNEL(name, d)                                                               \
+// From three activation rows on the four CTAs of a cluster share the staging of x (dd_body, CS = 4): every CTA used to
+// quantize all m x 16 (row, unit) pairs of a K = 4096 activation itself, eight per warp and about 11 us per op at
+// eight rows. 33 clusters of four run at once on a B200 (132 of 148 SMs; of two, 74): whole step of 32 layers at
+// eight rows 2.99 ms alone, 2.76 in twos, 2.60 in fours; 8 layers at four rows 624 us (barrier form with activation
+// images) -> 421, at three 405 -> 400; one and two rows have a pair or two per warp and stay alone.
+// n2: five to eight rows, two column tiles (D = 2 or 3 stages: sixteen limb planes take the room of the fourth).
+#define QM_DDX_KERNEL(name, d, nt)                                                           \
     extern "C" __global__ void __launch_bounds__(QM_GEMV_MAX_THREADS, 1)                     \
         name(const __grid_constant__ QmFusedArgs a) {                                        \
-        dd_body<2, d, false, false, 2>(a);                                                   \
+        dd_body<2, d, false, false, nt, 4>(a);                                               \
     }
-QM_DD8_KERNEL(qm_fused_q4k_dd_n2d2, 2)
-QM_DD8_KERNEL(qm_fused_q4k_dd_n2d3, 3)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d2_x4, 2, 1)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d3_x4, 3, 1)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d4_x4, 4, 1)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d2_x4, 2, 2)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d3_x4, 3, 2)
 
 // One activation row per op and ops whose matrix is chosen on the device from a table of experts
-// (QmOp::sel_table): decode-time MoE as a list of (token, slot) matvecs.
+// (QmOp::sel_table): decode-time MoE as a list of (token, slot) matvecs. Clusters of four share the staging (the down
+// ops' K is long: 56 units of a 14336-wide x are one per warp of a cluster instead of 3.5), and the ops' tiles start at
+// rotating CTAs: two tokens of eight 4096 x 14336 experts 148.2 -> 140 us (rotation alone 144).
 #define QM_DD_SEL_KERNEL(name, d)                                                            \
     extern "C" __global__ void __launch_bounds__(QM_GEMV_MAX_THREADS, 1)                     \
         name(const __grid_constant__ QmFusedArgs a) {                                        \
-        dd_body<4, d, false, true>(a);                                                       \
+        dd_body<4, d, false, true, 1, 4>(a);                                                 \
     }
 QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d2_sel, 2)
 QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d3_sel, 3)
@@ -1998,6 +2071,17 @@ QM_LEAN_KERNEL(qm_gemv_q80_lean_c2d3, 8, 2, 3, 1)
 QM_LEAN_KERNEL(qm_gemv_q80_lean_c2d2, 8, 2, 2, 1)
 QM_LEAN_KERNEL(qm_gemv_q80_lean_c2n2d3, 8, 2, 3, 2)
 QM_LEAN_KERNEL(qm_gemv_q80_lean_c2n2d2, 8, 2, 2, 2)
+
+// Seven and eight rows: two CTAs of a cluster share the staging of x (lean_body, CS = 2).
+#define QM_LEANX_KERNEL(name, fmt, d)                                                        \
+    extern "C" __global__ void __launch_bounds__(QM_GEMV_MAX_THREADS, 1)                     \
+        name(const __grid_constant__ QmLeanArgs a) {                                         \
+        lean_body<fmt, 2, d, 2, 2>(a);                                                       \
+    }
+QM_LEANX_KERNEL(qm_gemv_q40_lean_c2n2d4_x2, 2, 4)
+QM_LEANX_KERNEL(qm_gemv_q40_lean_c2n2d2_x2, 2, 2)
+QM_LEANX_KERNEL(qm_gemv_q80_lean_c2n2d3_x2, 8, 3)
+QM_LEANX_KERNEL(qm_gemv_q80_lean_c2n2d2_x2, 8, 2)
 
 // out[j][r] = c_j * sum over the K parts of a lean matvec, c_j = rsqrt(mean square + eps) from the parts' sums of
 // squares when the matvec normalises its input, else 1.

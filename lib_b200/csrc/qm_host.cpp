@@ -113,7 +113,10 @@ static const KernelName kKernels[QM_K_COUNT] = {
     {QM_MOD_Q4K, "qm_gemv_q80_lean_c4d3"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c4d2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2d3"},
     {QM_MOD_Q4K, "qm_gemv_q80_lean_c2d2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d3"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2"},
     {QM_MOD_Q4K, "qm_lean_sum"},
-    {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3"},
+    {QM_MOD_Q4K, "qm_gemv_q40_lean_c2n2d4_x2"}, {QM_MOD_Q4K, "qm_gemv_q40_lean_c2n2d2_x2"},
+    {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d3_x2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2_x2"},
+    {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d3_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d4_x4"},
+    {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3_x4"},
 };
 
 // ---- errors --------------------------------------------------------------------------
@@ -203,7 +206,7 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
                 r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
-        for (int k = QM_K_FUSED_Q4K_DD_N2D2; k <= QM_K_FUSED_Q4K_DD_N2D3 && !err; k++) {
+        for (int k = QM_K_Q40_LEAN_X2_D4; k <= QM_K_DD_X4_N2D3 && !err; k++) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
@@ -226,6 +229,10 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
         for (int cg = 1; cg <= 2 && !err; cg++)
             for (int k = 1; k <= 4; k *= 2)
                 c->gemm_clusters[cg - 1][k] = qm_max_clusters(c, cg == 2 ? QM_K_GEMM_PAIR : QM_K_GEMM_SOLO, cg * k, 768, QM_GEMV_SMEM_MAX);
+        if (!err) {
+            c->max_clusters[2] = qm_max_clusters(c, QM_K_Q40_LEAN_X2_D4, 2, 512, QM_GEMV_SMEM_MAX);
+            c->max_clusters[4] = qm_max_clusters(c, QM_K_DD_X4_N2D3, 4, 512, QM_GEMV_SMEM_MAX);
+        }
         if (!err) {
             r = d->cuStreamCreate(&c->own_stream, CU_STREAM_NON_BLOCKING);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
@@ -902,17 +909,24 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
         const bool q40 = w->fmt == QM_FMT_Q4_0;
         const int cpm = m <= 2 ? 4 : 2, nt = m <= 4 ? 1 : 2, planes = m * (cpm == 4 ? 3 : 2);
         const int stage = (q40 ? 2048 : 4096) + 256;
-        const int grid = qm_fused_grid(c), tiles = (int)((w->rows + 15) / 16);
+        // Seven or eight rows: two CTAs of a cluster share the staging of x, 3.5 or 4 (row, unit) pairs per warp of a
+        // K = 4096 matvec each instead of 7 or 8. 14336 x 4096 at eight rows: Q4_0 20.6 -> 18.6 us, Q8_0 24.4 -> 22.7;
+        // at five rows no gain (Q8_0 21.0 -> 22.4), nor where a long K runs in parts (22.5 us either way), and
+        // clusters of four leave 16 SMs idle (20.5 / 23.3 us).
+        const bool may_share = m >= 7 && c->max_clusters[2] * 2 >= qm_fused_grid(c);
+        const int tiles = (int)((w->rows + 15) / 16);
         const int64_t ldp = (w->rows + 3) & ~(int64_t)3;
         const int want = env_int("QM_LEAN_PARTS", w->units >= 32 ? 4 : 1);
         const int order[3] = {want, want == 4 ? 2 : want == 2 ? 4 : 2, want == 1 ? 4 : 1};
         const int depths[2] = {q40 ? 4 : 3, 2};
         for (int oi = 0; oi < 3; oi++) {
             const int S = order[oi];
-            if (S < 1 || w->units % S != 0 || grid % S != 0) continue;
+            if (S < 1 || w->units % S != 0) continue;
+            const int share = may_share && S == 1 && qm_fused_grid(c) % 2 == 0 ? 2 : 1, grid = qm_fused_grid(c);
+            if (grid % S != 0) continue;
             if (S > 1 && (!partials || 256 + (int64_t)S * m * ldp * 4 > QM_PARTIALS_BYTES)) continue;
             const int ups = w->units / S;
-            const int64_t fixed = (int64_t)planes * (ups * 256 + 64) + (int64_t)ups * nt * 160 + 512 + 16 * 2 * m * 64 + 128;
+            const int64_t fixed = (int64_t)planes * (ups * 256 + 64) + (int64_t)ups * nt * 160 + 512 * share + 16 * 2 * m * 64 + 128;
             for (int di = 0; di < 2; di++) {
                 const int64_t smem = fixed + (int64_t)16 * depths[di] * stage;
                 if (smem > QM_GEMV_SMEM_MAX) continue;
@@ -944,9 +958,10 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
                     la.ldy = ldp;
                     la.part_stride = (int64_t)m * ldp;
                 }
-                const int k = (q40 ? QM_K_Q40_LEAN_C4D4 : QM_K_Q80_LEAN_C4D3) + (cpm == 4 ? 0 : nt == 1 ? 2 : 4) + di;
+                const int k = share == 2 ? (q40 ? QM_K_Q40_LEAN_X2_D4 : QM_K_Q80_LEAN_X2_D3) + di
+                                         : (q40 ? QM_K_Q40_LEAN_C4D4 : QM_K_Q80_LEAN_C4D3) + (cpm == 4 ? 0 : nt == 1 ? 2 : 4) + di;
                 const bool pdl = (flags & QM_FLAG_PDL) != 0;
-                int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, pdl, false);
+                int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, pdl, false, share);
                 if (lrc || S == 1) return lrc;
                 QmSumPartsArgs sa;
                 memset(&sa, 0, sizeof sa);

@@ -28,7 +28,8 @@ enum {
     QM_K_EP_PUSH, QM_K_EP_COLLECT, QM_K_EP_RETURN, QM_K_EP_COMBINE,
     QM_K_Q40_LEAN_C4D4, QM_K_Q40_LEAN_C4D2, QM_K_Q40_LEAN_C2D4, QM_K_Q40_LEAN_C2D2, QM_K_Q40_LEAN_C2N2D4, QM_K_Q40_LEAN_C2N2D2,
     QM_K_Q80_LEAN_C4D3, QM_K_Q80_LEAN_C4D2, QM_K_Q80_LEAN_C2D3, QM_K_Q80_LEAN_C2D2, QM_K_Q80_LEAN_C2N2D3, QM_K_Q80_LEAN_C2N2D2,
-    QM_K_LEAN_SUM, QM_K_FUSED_Q4K_DD_N2D2, QM_K_FUSED_Q4K_DD_N2D3, QM_K_COUNT
+    QM_K_LEAN_SUM, QM_K_Q40_LEAN_X2_D4, QM_K_Q40_LEAN_X2_D2, QM_K_Q80_LEAN_X2_D3, QM_K_Q80_LEAN_X2_D2,
+    QM_K_DD_X4_C2D2, QM_K_DD_X4_C2D3, QM_K_DD_X4_C2D4, QM_K_DD_X4_N2D2, QM_K_DD_X4_N2D3, QM_K_COUNT
 };
 
 #define QM_GEMV_SMEM_MAX (227 * 1024)
@@ -47,6 +48,7 @@ struct qm_ctx {
     int sm_count, l2_bytes;
     CUmodule modules[QM_MOD_COUNT];
     int gemm_clusters[2][5];   // [CTAs per tile - 1][K shares]: clusters of the matmul by CTA pairs that run at once
+    int max_clusters[5];   // clusters of 2 and 4 GEMV CTAs (512 threads, all of the shared memory) that run at once
     CUfunction fn[QM_K_COUNT];
     CUstream own_stream, stream;
     CUdeviceptr status_dev, tickets_dev, partials_dev, gridbar_dev;

@@ -133,7 +133,7 @@ struct alignas(16) QmOp {   // a multiple of 16 bytes: the kernels copy descript
     // to every GPU's arena.
     float *y2;
     int32_t split_row;
-    int32_t pad3_;
+    int32_t cta_rot;     // *_sel kernels: CTA c is the op's (c + cta_rot) mod nctas -th, see dd_body
 };
 
 struct QmFusedArgs {

@@ -347,6 +347,7 @@ struct qm_moe_decode {
     CUdeviceptr ops_dev;
     CUdeviceptr sync;
     QmFusedPlan plan;
+    int grid;                // CTAs of the launch, in clusters of four
     int kernel;
     // what the device op list was built for
     int built_tokens;
@@ -411,6 +412,11 @@ extern "C" int32_t qm_moe_decode_create(qm_ctx *c, const qm_weight *gate_up, con
         delete d;
         return QM_ERR_SHAPE;
     }
+    d->grid = c->max_clusters[4] * 4;
+    if (d->grid < 4) {
+        delete d;
+        return QM_ERR_SHAPE;
+    }
     d->kernel = QM_K_FUSED_Q4K_DD_C4D2_SEL + (d->plan.depth - 2);
     CtxGuard g(c);
     if (g.rc != CUDA_SUCCESS) {
@@ -452,6 +458,14 @@ extern "C" int32_t qm_moe_decode_run(qm_ctx *c, qm_moe_decode *d, uint64_t x_dev
     if (tokens != d->built_tokens || x_dev != d->built_x || ids_dev != d->built_ids || ldx != d->built_ldx) {
         // all gate|up ops first: by the time a pair's down op stages its x, that x has long been written
         std::vector<QmOp> ops((size_t)2 * pairs);
+        int64_t dealt = 0;   // tiles beyond whole rounds of the CTAs, over all ops so far
+        auto deal = [&](QmOp &op) {   // the CTAs with one tile more follow those of the op before
+            op.nctas = d->grid;
+            op.q = op.tiles / d->grid;
+            op.rem = op.tiles % d->grid;
+            op.cta_rot = (int32_t)((d->grid - dealt % d->grid) % d->grid);
+            dealt += op.rem;
+        };
         for (int pr = 0; pr < pairs; pr++) {
             const int t = pr / d->topk;
             QmOp &a = ops[pr], &b = ops[pairs + pr];
@@ -465,7 +479,9 @@ extern "C" int32_t qm_moe_decode_run(qm_ctx *c, qm_moe_decode *d, uint64_t x_dev
             a.sel_ids = b.sel_ids = (const int32_t *)(uintptr_t)ids_dev;
             a.sel_index = b.sel_index = pr;
             a.sel_count = b.sel_count = d->experts;
+            deal(a);
         }
+        for (int pr = 0; pr < pairs; pr++) deal(ops[pairs + pr]);
         DRV(c->drv->cuStreamSynchronize(c->stream));   // the list in use may still be read
         DRV(c->drv->cuMemcpyHtoD_v2(d->ops_dev, ops.data(), ops.size() * sizeof(QmOp)));
         d->built_tokens = tokens;
@@ -492,8 +508,8 @@ extern "C" int32_t qm_moe_decode_run(qm_ctx *c, qm_moe_decode *d, uint64_t x_dev
     a.wait_cycles = qm_wait_cycles();
     // no programmatic launch: the ids must be complete before the first copy is issued; cooperative: the CTAs
     // poll one another's outputs and must all be resident
-    int32_t rc = qm_launch_ex(c, d->kernel, (unsigned)qm_fused_grid(c), (unsigned)d->plan.consumers * 32,
-                              (unsigned)d->plan.smem, &a, false, true);
+    int32_t rc = qm_launch_ex(c, d->kernel, (unsigned)d->grid, (unsigned)d->plan.consumers * 32,
+                              (unsigned)d->plan.smem, &a, false, true, 4);
     if (rc) return rc;
     QmDecodeCombineArgs ca;
     memset(&ca, 0, sizeof ca);

@@ -54,6 +54,7 @@ struct qm_stack {
     int fused_dd_kernel[9];
     int fused_half0[9];         // tensor-parallel: arena half that the first copy of the op list addresses
     int fused_parts_o[9], fused_parts_dn[9];   // K parts of the o / down projections in the op list (1 = whole)
+    int fused_share[9], fused_grid[9];   // CTAs of a cluster that share a staging (1: none), CTAs of the launch
     int fused_ngroups[9];       // CTA groups with a copy of the op list each (data-driven form with K parts)
     // tensor-parallel: one arena holds all activation buffers and the peers' arrival flags; the
     // peers map it through CUDA IPC and this GPU stores its row slices into all of them
@@ -459,10 +460,13 @@ static int32_t part_major_copy(qm_ctx *c, const QmWeight *w, int parts, CUdevice
 }
 
 static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
-    // up to three rows, and five to eight (two column tiles; single GPU); four rows run with activation images
-    const bool two_tiles = m > 4 && s->tp_world == 1 && qm_env_int("QM_DD8", 1) != 0;
-    if ((m >= qm_env_int("QM_IMAGE_MIN_M", 4) && !two_tiles) || qm_env_int("QM_DD", 1) == 0) return QM_ERR_SHAPE;
-    const int grid = qm_fused_grid(c);
+    // Single GPU: every batch; from three rows on the CTAs of a cluster of four share the staging of x (both sides
+    // measured beside the kernels, qm_fused_q4k_dd_*_x4). Tensor parallel: up to three rows.
+    const bool tp_list = s->tp_world > 1;
+    if (m >= qm_env_int("QM_IMAGE_MIN_M", tp_list ? 4 : 9) || qm_env_int("QM_DD", 1) == 0) return QM_ERR_SHAPE;
+    const int share = m >= 3 && !tp_list && c->max_clusters[4] >= QM_MAX_PARTS ? 4 : 1;
+    if (m >= 4 && share == 1 && !tp_list) return QM_ERR_SHAPE;
+    const int grid = share > 1 ? c->max_clusters[share] / QM_MAX_PARTS * QM_MAX_PARTS * share : qm_fused_grid(c);
     // The down projection (long K: its CTAs would each quantize all 2 x 14336 activations) runs in
     // four K parts. The o projection stays whole by default: its x is short, and every part adds a
     // vector that each CTA of the consumer polls and loads.
@@ -490,13 +494,13 @@ static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
     if (qm_plan_fused(c, m, max_units, false, &p) != QM_OK) return QM_ERR_SHAPE;
     int kernel = -1;
     if (p.nt == 1 && p.consumers == 16 && p.depth >= 2 && p.depth <= 4)
-        kernel = (p.cpm == 4 ? QM_K_FUSED_Q4K_DD_C4D2 : QM_K_FUSED_Q4K_DD_C2D2) + (p.depth - 2);
+        kernel = (share == 4 ? QM_K_DD_X4_C2D2 : p.cpm == 4 ? QM_K_FUSED_Q4K_DD_C4D2 : QM_K_FUSED_Q4K_DD_C2D2) + (p.depth - 2);
     if (p.nt == 2 && p.consumers == 16 && p.depth >= 2) {
         if (p.depth > 3) {   // the two-tile kernels exist with two and three stages
             p.smem -= (p.depth - 3) * 16 * QM_Q4K_ITEM_BYTES;
             p.depth = 3;
         }
-        kernel = QM_K_FUSED_Q4K_DD_N2D2 + (p.depth - 2);
+        kernel = QM_K_DD_X4_N2D2 + (p.depth - 2);
     }
     if (kernel < 0) return QM_ERR_SHAPE;
     for (int L = 0; L < s->layers; L++) {
@@ -521,6 +525,9 @@ static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
             QmOp op;
             const int ups = w->units / parts;
             qm_fill_op(c, p, w, x, x2, ldx, y + R * w->rows, ldy, xop, !first, 0, ups, 0, &op);
+            op.nctas = grid;
+            op.q = op.tiles / grid;
+            op.rem = op.tiles % grid;
             if (parts > 1) {
                 const int per = ngroups / parts;          // CTA groups that share one part
                 const int part = g / per, G = grid / ngroups * per;
@@ -581,6 +588,8 @@ static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
     s->fused_img[m] = false;
     s->fused_dd[m] = true;
     s->fused_dd_kernel[m] = kernel;
+    s->fused_share[m] = share;
+    s->fused_grid[m] = grid;
     s->fused_parts_o[m] = So;
     s->fused_parts_dn[m] = Sd;
     s->fused_plan[m] = p;
@@ -917,8 +926,8 @@ static int32_t launch_fused(qm_ctx *c, qm_stack *s, int m) {
         // every output word of the step starts as "not yet written" (all ones)
         const size_t bytes = (size_t)(layer_bufs(s, s->layers, m).qkv - s->act);
         DRV(c->drv->cuMemsetD32Async(s->act, 0xFFFFFFFFu, bytes / 4, c->stream));
-        int32_t rc = qm_launch_ex(c, s->fused_dd_kernel[m], (unsigned)qm_fused_grid(c), (unsigned)p.consumers * 32,
-                                  (unsigned)p.smem, &a, false, true);
+        int32_t rc = qm_launch_ex(c, s->fused_dd_kernel[m], (unsigned)s->fused_grid[m], (unsigned)p.consumers * 32,
+                                  (unsigned)p.smem, &a, false, true, s->fused_share[m]);
         return rc ? rc : sum_last_parts(c, s, m);
     }
     const int kern = s->fused_img[m] ? (p.nt == 1 ? QM_K_FUSED_Q4K_NT1_IMG : QM_K_FUSED_Q4K_NT2_IMG)

@@ -1,0 +1,77 @@
+"""GPU parity of the kernels that run in thread-block clusters, at the sizes where they can go wrong: the matmul by CTA
+pairs (row tiles, token tiles, K shares), the eight-row Q4_0 / Q8_0 matvecs and the decode step whose CTAs share the
+staging of x; and of the one-row Q8_1 matvecs with the activations in registers."""
+import numpy as np
+import pytest
+
+import lib_b200
+from lib_b200 import _capi, synth
+from oracle import oracle
+from tests import q8_1_cases as cases
+from tests.test_gpu_matmul import TOL as MATMUL_TOL, run as run_matmul
+from tests.test_gpu_stack import build_stack, nre, oracle_chain
+
+pytestmark = pytest.mark.gpu
+
+
+# Rows around one CTA's 128 and a pair's 256; tokens around the rounding to 16, a tile of 32 and the largest tiles;
+# one K unit, fewer units than K shares, more units than the ring of weight items; many row tiles (no split, several
+# rounds per pair).
+@pytest.mark.parametrize("n,k,m", [(1, 256, 1), (127, 256, 15), (129, 512, 17), (255, 768, 32), (257, 1024, 33), (256, 2560, 127),
+                                   (640, 5120, 129), (272, 256, 255), (520, 512, 257), (144, 2304, 481), (20000, 256, 31),
+                                   (9500, 512, 161)])
+def test_matmul_edges(ctx, devbuf, n, k, m):
+    assert run_matmul(ctx, devbuf, n, k, m, seed=3 * n + m) <= MATMUL_TOL
+
+
+# Two limbs per activation row from three rows on: 14 bits of the unit's maximum, 3e-4 normwise (as in the matvec
+# tests). K of one unit, a partial unit, an odd number of units, and a long K that runs in parts.
+@pytest.mark.parametrize("fmt", [2, 8])
+@pytest.mark.parametrize("m", [6, 7, 8])
+@pytest.mark.parametrize("rows,cols,xop", [(16, 256, 0), (33, 288, 1), (2400, 2336, 1), (4736, 1280, 0), (96, 8192, 1)])
+def test_matvec_shared_staging(ctx, devbuf, fmt, m, rows, cols, xop):
+    raw = synth.weights(fmt, rows, cols, seed=rows + m)
+    w = ctx.store_upload(fmt, rows, cols, raw)
+    x = synth.activations(m, cols, 9)
+    yd = devbuf(np.full((m, rows), np.nan, np.float32))
+    ctx.matvec(w, devbuf(x).ptr, m, cols, yd.ptr, rows, xop)
+    got = yd.get((m, rows))
+    assert ctx.last_status() == (0, 0)
+    want = oracle.MatVec(fmt, raw, rows, cols, oracle.RMSNorm(x) if xop else x)
+    assert nre(got, want) <= 3e-4
+    w.free()
+
+
+# Hidden sizes of fewer units than the cluster has warps, an odd number of units, and a down projection that cannot be
+# cut into four parts (5 and 7 units) or can (8).
+@pytest.mark.parametrize("m", [3, 4, 6, 7, 8])
+@pytest.mark.parametrize("hidden,kv,ffn", [(256, 32, 1280), (768, 96, 1792), (1280, 160, 2048)])
+def test_step_shared_staging(ctx, m, hidden, kv, ffn):
+    st, raws = build_stack(ctx, 2, hidden, kv, ffn, 12, seed=41)
+    x = synth.activations(m, hidden, 8)
+    h, kvs = st.step_host(x, want_kv=True)
+    want_h, want_kv, _ = oracle_chain(12, raws, x, hidden, kv, ffn)
+    assert nre(h, want_h) <= 1e-3 and nre(kvs, want_kv) <= 1e-3
+    assert np.array_equal(h, st.step_host(x))
+    st.close()
+
+
+# Steps of four super-blocks: a single one, whole steps, a remainder, the largest K in registers and the first beyond.
+# (Rows of Q2_K / IQ2_XXS are whole 16-byte pieces, which the staged form needs, at multiples of four / eight units.)
+@pytest.mark.parametrize("fmt", [10, 16])
+@pytest.mark.parametrize("cols", [256, 1024, 2048, 3072, 4096, 6144])
+def test_q8_1_row(ctx, devbuf, fmt, cols):
+    experts, rows = 3, 41
+    raw = synth.weights(fmt, experts * rows, cols, seed=fmt + cols)
+    w = ctx.store_upload(fmt, experts * rows, cols, raw)
+    ids = np.array([2, 7, 0], dtype=np.int32)
+    x, _ = cases.random_rows(1, cols, seed=cols)
+    xq = oracle.RMSNormQ8_1(x, None, 1, cols, 1e-6, False)
+    xd, yd = devbuf(np.frombuffer(xq, dtype=np.uint8)), devbuf(nbytes=len(ids) * rows * 4)
+    ctx.matvec_selected(w, experts, devbuf(ids).ptr, len(ids), xd.ptr, 0, yd.ptr, _capi.FLAG_X_Q8_1)
+    got = yd.get((len(ids), rows))
+    want = oracle.SelectedMatVecQ8_1(fmt, raw, experts, rows, cols, [2, -1, 0], xq)
+    # exact integer sums per group, float32 across groups: 2e-5 of the largest output, as for the other Q8_1 matvecs
+    assert np.abs(got[[0, 2]] - want[[0, 2]]).max() <= 2e-5 * np.abs(want[[0, 2]]).max()
+    assert np.all(got[1].view(np.uint32) == 0x7fffffff)
+    w.free()
