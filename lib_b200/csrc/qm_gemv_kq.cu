@@ -498,10 +498,7 @@ __device__ __forceinline__ void gemv_kq_q81_row1(const QmKqArgs &a, uint32_t *ta
 // and for Q8_1 activations.
 #define QM_KQ_KERNEL(name, fmt, mm, xq)                                                                        \
     extern "C" __global__ void __launch_bounds__(256) name(const __grid_constant__ QmKqArgs a) {               \
-        __shared__ uint32_t tab[xq && mm == 1 && fmt == 16 ? 384 * kCopies : 1];                               \
-        if (xq && mm == 1 && a.depth >= 2 && a.units <= 8) gemv_kq_q81_row1<fmt, 2>(a, tab);                   \
-        else if (xq && mm == 1 && a.depth >= 2 && a.units <= 16) gemv_kq_q81_row1<fmt, 4>(a, tab);             \
-        else if (a.depth >= 2) gemv_kq_body<fmt, mm, xq, true>(a);                                             \
+        if (a.depth >= 2) gemv_kq_body<fmt, mm, xq, true>(a);                                                  \
         else gemv_kq_body<fmt, mm, xq, false>(a);                                                              \
     }
 QM_KQ_KERNEL(qm_gemv_q2k_m1, 10, 1, false)
@@ -520,3 +517,14 @@ QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m1, 16, 1, true)
 QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m2, 16, 2, true)
 QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m4, 16, 4, true)
 QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m8, 16, 8, true)
+
+// One Q8_1 row through the staged form, K up to 4096 (kernels of their own: the registers that hold the activations
+// would cost the direct form its occupancy; with one entry for both it lost up to 10 %).
+#define QM_KQ_ROW_KERNEL(name, fmt)                                                                            \
+    extern "C" __global__ void __launch_bounds__(256) name(const __grid_constant__ QmKqArgs a) {               \
+        __shared__ uint32_t tab[fmt == 16 ? 384 * kCopies : 1];                                                \
+        if (a.units <= 8) gemv_kq_q81_row1<fmt, 2>(a, tab);                                                    \
+        else gemv_kq_q81_row1<fmt, 4>(a, tab);                                                                 \
+    }
+QM_KQ_ROW_KERNEL(qm_gemv_q2k_q81_row, 10)
+QM_KQ_ROW_KERNEL(qm_gemv_iq2xxs_q81_row, 16)

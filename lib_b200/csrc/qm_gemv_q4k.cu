@@ -1998,35 +1998,37 @@ QM_DD_KERNEL(qm_fused_q4k_dd_c2d2_tp, 2, 2, true)
 QM_DD_KERNEL(qm_fused_q4k_dd_c2d3_tp, 2, 3, true)
 QM_DD_KERNEL(qm_fused_q4k_dd_c2d4_tp, 2, 4, true)
 
-// From three activation rows on the four CTAs of a cluster share the staging of x (dd_body, CS = 4): every CTA used to
-// quantize all m x 16 (row, unit) pairs of a K = 4096 activation itself, eight per warp and about 11 us per op at
-// eight rows. 33 clusters of four run at once on a B200 (132 of 148 SMs; of two, 74): whole step of 32 layers at
-// eight rows 2.99 ms alone, 2.76 in twos, 2.60 in fours; 8 layers at four rows 624 us (barrier form with activation
-// images) -> 421, at three 405 -> 400; one and two rows have a pair or two per warp and stay alone.
-// n2: five to eight rows, two column tiles (D = 2 or 3 stages: sixteen limb planes take the room of the fourth).
-#define QM_DDX_KERNEL(name, d, nt)                                                           \
+// Five to eight activation rows: two column tiles (D = 2 or 3 stages: sixteen limb planes take the room of the fourth).
+// *_x4: the four CTAs of a cluster share the staging of x (CS = 4). A CTA alone quantizes all m x units (row, unit)
+// pairs of an activation itself, eight per warp and about 11 us per op at eight rows of K = 4096. A cluster costs two
+// barriers per op and 16 SMs: 33 clusters of four run at once on a B200 (132 of 148 SMs; of two, 74). Whole step of 32
+// layers at eight rows: 2.99 ms alone, 2.76 in twos, 2.60 in fours; the host's rule (build_fused_dd) has the rest.
+#define QM_DDX_KERNEL(name, d, nt, cs)                                                       \
     extern "C" __global__ void __launch_bounds__(QM_GEMV_MAX_THREADS, 1)                     \
         name(const __grid_constant__ QmFusedArgs a) {                                        \
-        dd_body<2, d, false, false, nt, 4>(a);                                               \
+        dd_body<2, d, false, false, nt, cs>(a);                                              \
     }
-QM_DDX_KERNEL(qm_fused_q4k_dd_c2d2_x4, 2, 1)
-QM_DDX_KERNEL(qm_fused_q4k_dd_c2d3_x4, 3, 1)
-QM_DDX_KERNEL(qm_fused_q4k_dd_c2d4_x4, 4, 1)
-QM_DDX_KERNEL(qm_fused_q4k_dd_n2d2_x4, 2, 2)
-QM_DDX_KERNEL(qm_fused_q4k_dd_n2d3_x4, 3, 2)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d2, 2, 2, 1)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d3, 3, 2, 1)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d2_x4, 2, 1, 4)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d3_x4, 3, 1, 4)
+QM_DDX_KERNEL(qm_fused_q4k_dd_c2d4_x4, 4, 1, 4)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d2_x4, 2, 2, 4)
+QM_DDX_KERNEL(qm_fused_q4k_dd_n2d3_x4, 3, 2, 4)
 
 // One activation row per op and ops whose matrix is chosen on the device from a table of experts
-// (QmOp::sel_table): decode-time MoE as a list of (token, slot) matvecs. Clusters of four share the staging (the down
-// ops' K is long: 56 units of a 14336-wide x are one per warp of a cluster instead of 3.5), and the ops' tiles start at
-// rotating CTAs: two tokens of eight 4096 x 14336 experts 148.2 -> 140 us (rotation alone 144).
-#define QM_DD_SEL_KERNEL(name, d)                                                            \
+// (QmOp::sel_table): decode-time MoE as a list of (token, slot) matvecs.
+#define QM_DD_SEL_KERNEL(name, d, cs)                                                        \
     extern "C" __global__ void __launch_bounds__(QM_GEMV_MAX_THREADS, 1)                     \
         name(const __grid_constant__ QmFusedArgs a) {                                        \
-        dd_body<4, d, false, true, 1, 4>(a);                                                 \
+        dd_body<4, d, false, true, 1, cs>(a);                                                \
     }
-QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d2_sel, 2)
-QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d3_sel, 3)
-QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d4_sel, 4)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d2_sel, 2, 1)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d3_sel, 3, 1)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d4_sel, 4, 1)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d2_sel_x4, 2, 4)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d3_sel_x4, 3, 4)
+QM_DD_SEL_KERNEL(qm_fused_q4k_dd_c4d4_sel_x4, 4, 4)
 
 // h = c * (sum of the K parts of the step's last matvec), see QmSumPartsArgs.
 extern "C" __global__ void __launch_bounds__(256) qm_sum_parts(const __grid_constant__ QmSumPartsArgs a) {

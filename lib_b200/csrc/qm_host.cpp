@@ -103,8 +103,10 @@ static const KernelName kKernels[QM_K_COUNT] = {
     {QM_MOD_KQ, "qm_gemv_q2k_q81_m1"}, {QM_MOD_KQ, "qm_gemv_q2k_q81_m2"}, {QM_MOD_KQ, "qm_gemv_q2k_q81_m4"},
     {QM_MOD_KQ, "qm_gemv_q2k_q81_m8"}, {QM_MOD_KQ, "qm_gemv_iq2xxs_q81_m1"}, {QM_MOD_KQ, "qm_gemv_iq2xxs_q81_m2"},
     {QM_MOD_KQ, "qm_gemv_iq2xxs_q81_m4"}, {QM_MOD_KQ, "qm_gemv_iq2xxs_q81_m8"},
+    {QM_MOD_KQ, "qm_gemv_q2k_q81_row"}, {QM_MOD_KQ, "qm_gemv_iq2xxs_q81_row"},
     {QM_MOD_Q81, "qm_rmsnorm_q8_1"},   {QM_MOD_Q81, "qm_swiglu_q8_1"},    {QM_MOD_Q81, "qm_q8_1_expand"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d2_sel"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d3_sel"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d4_sel"},
+    {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d2_sel_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d3_sel_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c4d4_sel_x4"},
     {QM_MOD_MOE, "qm_moe_decode_combine"},
     {QM_MOD_MOE, "qm_ep_push"},        {QM_MOD_MOE, "qm_ep_collect"},     {QM_MOD_MOE, "qm_ep_return"},
     {QM_MOD_MOE, "qm_ep_combine"},
@@ -117,6 +119,7 @@ static const KernelName kKernels[QM_K_COUNT] = {
     {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d3_x2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2_x2"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d3_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d4_x4"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3_x4"},
+    {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3"},
 };
 
 // ---- errors --------------------------------------------------------------------------
@@ -206,7 +209,7 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
                 r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
-        for (int k = QM_K_Q40_LEAN_X2_D4; k <= QM_K_DD_X4_N2D3 && !err; k++) {
+        for (int k = QM_K_Q40_LEAN_X2_D4; k <= QM_K_FUSED_Q4K_DD_N2D3 && !err; k++) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
@@ -214,11 +217,11 @@ extern "C" int32_t qm_init(int32_t device, qm_ctx **out) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
-        for (int k = QM_K_FUSED_Q4K_DD_C4D2_SEL; k <= QM_K_FUSED_Q4K_DD_C4D4_SEL && !err; k++) {
+        for (int k = QM_K_FUSED_Q4K_DD_C4D2_SEL; k <= QM_K_DD_X4_SEL_D4 && !err; k++) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_GEMV_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
-        for (int k = QM_K_GEMV_Q2K_M1; k <= QM_K_GEMV_IQ2XXS_Q81_M8 && !err; k++) {
+        for (int k = QM_K_GEMV_Q2K_M1; k <= QM_K_GEMV_IQ2XXS_Q81_ROW && !err; k++) {
             r = d->cuFuncSetAttribute(c->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, QM_KQ_SMEM_MAX);
             if (r != CUDA_SUCCESS) err = (int32_t)r;
         }
@@ -854,8 +857,8 @@ int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int3
     ka.x_slot_stride = x_slot_stride;
     ka.y_slot_stride = ids_dev ? ka.rows : 0;
     const int mi = m <= 1 ? 0 : m <= 2 ? 1 : m <= 4 ? 2 : 3;
-    const int k = (w->fmt == QM_FMT_Q2_K ? (xq ? QM_K_GEMV_Q2K_Q81_M1 : QM_K_GEMV_Q2K_M1)
-                                         : (xq ? QM_K_GEMV_IQ2XXS_Q81_M1 : QM_K_GEMV_IQ2XXS_M1)) + mi;
+    int k = (w->fmt == QM_FMT_Q2_K ? (xq ? QM_K_GEMV_Q2K_Q81_M1 : QM_K_GEMV_Q2K_M1)
+                                   : (xq ? QM_K_GEMV_IQ2XXS_Q81_M1 : QM_K_GEMV_IQ2XXS_M1)) + mi;
     // eight warps per CTA, one row per warp at a time. Rows that are whole 16-byte pieces are streamed through
     // per-warp rings in shared memory (2..4 rows in flight per warp, at most 96 KB per CTA); other shapes are
     // read with direct loads.
@@ -869,6 +872,9 @@ int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int3
             ka.depth = (int32_t)d;
             ka.xs_bytes = (int32_t)xs;
             smem = (unsigned)(xs + 8 * d * row_bytes);
+            // one Q8_1 row: the activations stay in registers up to K = 4096 (6 slots of 2048 x 4096 experts, the layer
+            // of gate, up and down matvecs and its producers: 62.6 -> 57.5 us)
+            if (xq && m == 1 && w->units <= 16) k = w->fmt == QM_FMT_Q2_K ? QM_K_GEMV_Q2K_Q81_ROW : QM_K_GEMV_IQ2XXS_Q81_ROW;
         }
     }
     const int per_sm = smem ? (int)std::max<int64_t>(1, std::min<int64_t>(8, (200 * 1024) / (smem + 3072))) : 8;

@@ -460,12 +460,17 @@ static int32_t part_major_copy(qm_ctx *c, const QmWeight *w, int parts, CUdevice
 }
 
 static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
-    // Single GPU: every batch; from three rows on the CTAs of a cluster of four share the staging of x (both sides
-    // measured beside the kernels, qm_fused_q4k_dd_*_x4). Tensor parallel: up to three rows.
+    // Single GPU: every batch. Tensor parallel: up to three rows.
     const bool tp_list = s->tp_world > 1;
     if (m >= qm_env_int("QM_IMAGE_MIN_M", tp_list ? 4 : 9) || qm_env_int("QM_DD", 1) == 0) return QM_ERR_SHAPE;
-    const int share = m >= 3 && !tp_list && c->max_clusters[4] >= QM_MAX_PARTS ? 4 : 1;
-    if (m >= 4 && share == 1 && !tp_list) return QM_ERR_SHAPE;
+    // Clusters of four share the staging of x where a CTA alone would quantize about three (row, unit) pairs of the
+    // hidden state per warp; below that their barriers and the 16 SMs they leave idle cost more. Eight layers, alone
+    // -> shared, us: m = 8 hidden 4096 (128 pairs) 796 -> 703, 2048 (64) 456 -> 419, 1280 (40) 440 -> 414; m = 6 4096
+    // (96) 646 -> 615, 2048 (48) 392 -> 384, 1280 (30) 350 -> 355; m = 5 3072 (60) 441 -> 417, 1280 (25) 325 -> 339;
+    // m = 4 4096 (64) 454 -> 420, 3072 (48) 350 -> 345, 2048 (32) 287 -> 304; m = 3 4096 405 -> 400, 1280 slower by a
+    // fifth. (Four rows as the barrier form with activation images: 624 at 4096, 401 at 2048, 352 at 1280.)
+    const int pairs = m * (int)(s->hidden / QM_K_UNIT);
+    const int share = !tp_list && m >= 4 && pairs >= (m >= 7 ? 35 : 48) && c->max_clusters[4] >= QM_MAX_PARTS ? 4 : 1;
     const int grid = share > 1 ? c->max_clusters[share] / QM_MAX_PARTS * QM_MAX_PARTS * share : qm_fused_grid(c);
     // The down projection (long K: its CTAs would each quantize all 2 x 14336 activations) runs in
     // four K parts. The o projection stays whole by default: its x is short, and every part adds a
@@ -500,7 +505,7 @@ static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
             p.smem -= (p.depth - 3) * 16 * QM_Q4K_ITEM_BYTES;
             p.depth = 3;
         }
-        kernel = QM_K_DD_X4_N2D2 + (p.depth - 2);
+        kernel = (share == 4 ? QM_K_DD_X4_N2D2 : QM_K_FUSED_Q4K_DD_N2D2) + (p.depth - 2);
     }
     if (kernel < 0) return QM_ERR_SHAPE;
     for (int L = 0; L < s->layers; L++) {
