@@ -230,6 +230,9 @@ __device__ __forceinline__ void gemv_kq_body(const QmKqArgs &a) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) grid[i] = QM_IQ2XXS_GRID_INIT[i];
         __syncthreads();
     }
+    // ids and x may come from the kernel before this one in the stream, which may still be running
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int kBlockBytes = FMT == 10 ? 84 : 66;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -366,6 +369,25 @@ __device__ __forceinline__ void gemv_kq_q81_row1(const QmKqArgs &a, uint32_t *ta
     const uint8_t *x = static_cast<const uint8_t *>(a.x) + (int64_t)slot * a.x_slot_stride * 36;
     const int64_t row_bytes = (int64_t)a.units * kBlockBytes;
     extern __shared__ __align__(16) uint8_t dyn_smem[];
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (FMT == 16) {
+        for (int i = threadIdx.x; i < 384; i += blockDim.x) {
+            uint32_t w = 0;
+            if (i < 256) {
+                const unsigned long long code = QM_IQ2XXS_GRID_INIT[i];
+#pragma unroll
+                for (int k = 0; k < 8; k++) w |= (uint32_t)((code >> (8 * k + 4)) & 3ull) << (4 * k);
+            } else {
+                const uint32_t si = i - 256, signs = si | ((uint32_t)(__popc(si) & 1) << 7);
+#pragma unroll
+                for (int k = 0; k < 8; k++) w |= ((signs >> k) & 1u) << (4 * k + 2);
+            }
+#pragma unroll
+            for (int k = 0; k < kCopies; k++) tab[i * kCopies + k] = w;
+        }
+    }
+    // ids and x may come from the kernel before this one in the stream, which may still be running
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (a.ids) {
         const int e = a.ids[slot];
         if (e < 0 || e >= a.experts) {
@@ -395,22 +417,6 @@ __device__ __forceinline__ void gemv_kq_q81_row1(const QmKqArgs &a, uint32_t *ta
     for (int d = 0; d < D; d++) issue();
     for (int i = threadIdx.x; i < a.units * 72; i += blockDim.x)
         reinterpret_cast<uint32_t *>(dyn_smem)[i] = __ldg(reinterpret_cast<const uint32_t *>(x) + i);
-    if (FMT == 16) {
-        for (int i = threadIdx.x; i < 384; i += blockDim.x) {
-            uint32_t w = 0;
-            if (i < 256) {
-                const unsigned long long code = QM_IQ2XXS_GRID_INIT[i];
-#pragma unroll
-                for (int k = 0; k < 8; k++) w |= (uint32_t)((code >> (8 * k + 4)) & 3ull) << (4 * k);
-            } else {
-                const uint32_t si = i - 256, signs = si | ((uint32_t)(__popc(si) & 1) << 7);
-#pragma unroll
-                for (int k = 0; k < 8; k++) w |= ((signs >> k) & 1u) << (4 * k + 2);
-            }
-#pragma unroll
-            for (int k = 0; k < kCopies; k++) tab[i * kCopies + k] = w;
-        }
-    }
     __syncthreads();
     const int i8 = lane & 7;   // the lane's Q8_1 block within its super-blocks
     int xw[STEPS][8];

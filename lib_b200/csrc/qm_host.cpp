@@ -480,6 +480,7 @@ extern "C" int32_t qm_store_create(qm_ctx *c, int32_t fmt, int64_t rows, int64_t
     if (fmt == QM_FMT_Q4_0) { qbytes = rows * w->units * 8 * 16; dbytes = rows * w->units * 8 * 2; }
     if (fmt == QM_FMT_Q8_0) { qbytes = rows * w->units * 8 * 32; dbytes = rows * w->units * 8 * 2; }
     w->qbytes = qbytes;
+    w->written = 1;   // the padding is zeroed in stream order
     w->dbytes = dbytes;
     CtxGuard g(c);
     CUresult r = g.rc;
@@ -500,7 +501,12 @@ extern "C" int32_t qm_store_create(qm_ctx *c, int32_t fmt, int64_t rows, int64_t
     return QM_OK;
 }
 
+bool qm_may_overlap(const QmWeight *w, uint32_t flags) {
+    return __atomic_exchange_n(&w->written, 0, __ATOMIC_RELAXED) == 0 || (flags & QM_FLAG_PDL) != 0;
+}
+
 static int32_t store_write_dev(qm_ctx *c, QmWeight *w, int64_t row_offset, int64_t nrows, CUdeviceptr src) {
+    __atomic_store_n(&w->written, 1, __ATOMIC_RELAXED);
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS) {
         DRV(c->drv->cuMemcpyDtoDAsync_v2(w->wq + row_offset * w->gguf_row_bytes, src,
                                          (size_t)(nrows * w->gguf_row_bytes), c->stream));
@@ -824,18 +830,19 @@ static int32_t fused_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev,
     a.debug_slot = env_int("QM_DEBUG_OP", 0);
 #endif
     a.wait_cycles = qm_wait_cycles();
+    const bool overlap = qm_may_overlap(w, flags);
     // One op of up to four activation rows whose K fits whole: the lean body of the data-driven
     // kernels (an op that reads the launch's input polls nothing).
     if (p.slices == 1 && p.nt == 1 && p.consumers == 16 && p.depth >= 2 && p.depth <= 4 && env_int("QM_DD", 1) != 0) {
         const int k = (p.cpm == 4 ? QM_K_FUSED_Q4K_DD_C4D2 : QM_K_FUSED_Q4K_DD_C2D2) + (p.depth - 2);
         return qm_launch_ex(c, k, (unsigned)qm_fused_grid(c), (unsigned)p.consumers * 32, (unsigned)p.smem, &a,
-                            (flags & QM_FLAG_PDL) != 0, false);
+                            overlap, false);
     }
     const bool coop = p.slices > 1;  // K slices meet at a grid barrier: all CTAs must be co-resident
     if (coop) DRV(c->drv->cuMemsetD32Async(c->gridbar_dev, 0, 1, c->stream));
     return qm_launch_ex(c, p.nt == 1 ? QM_K_FUSED_Q4K_NT1 : QM_K_FUSED_Q4K_NT2,
                         (unsigned)qm_fused_grid(c), (unsigned)p.consumers * 32, (unsigned)p.smem, &a,
-                        (flags & QM_FLAG_PDL) != 0 && !coop, coop);
+                        overlap && !coop, coop);
 }
 
 // Q2_K / IQ2_XXS: warp-per-row kernels over the GGUF bytes. x: float32 or (xq) Q8_1 blocks; ids_dev != 0: the
@@ -897,7 +904,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS) {
         // warp-per-row kernels over the GGUF bytes; plain products only (no fused input transform)
         if (xop != QM_XOP_NONE) return QM_ERR_ARG;
-        return qm_kq_launch(c, w, x_dev, false, m, ldx, y_dev, ldy, 0, 0, 1, 0, (flags & QM_FLAG_PDL) != 0);
+        return qm_kq_launch(c, w, x_dev, false, m, ldx, y_dev, ldy, 0, 0, 1, 0, qm_may_overlap(w, flags));
     }
     if (w->fmt == QM_FMT_Q4_K) {
         // integer tensor-core path; K is cut into slices when the activation planes of the
@@ -907,6 +914,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
         if (frc) return frc;
         return fused_matvec_launch(c, w, x_dev, x2_dev, m, ldx, y_dev, ldy, flags, fp);
     }
+    const bool pdl = qm_may_overlap(w, flags);
     if (env_int("QM_LEAN", 1) != 0) {
         // The integer tensor-core body: one persistent CTA of 16 warps per SM, whole tiles per CTA, per-warp
         // cp.async rings. A long K is cut into parts (CTA groups that each stage only their range of x and
@@ -919,7 +927,8 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
         // K = 4096 matvec each instead of 7 or 8. 14336 x 4096 at eight rows: Q4_0 20.6 -> 18.6 us, Q8_0 24.4 -> 22.7;
         // at five rows no gain (Q8_0 21.0 -> 22.4), nor where a long K runs in parts (22.5 us either way), and
         // clusters of four leave 16 SMs idle (20.5 / 23.3 us).
-        const bool may_share = m >= 7 && c->max_clusters[2] * 2 >= qm_fused_grid(c);
+        // Below six pairs per warp the cluster barriers cost more (28270 x 1376 at eight rows, three pairs: 17.3 -> 18.6).
+        const bool may_share = m >= 7 && m * w->units >= 96 && c->max_clusters[2] * 2 >= qm_fused_grid(c);
         const int tiles = (int)((w->rows + 15) / 16);
         const int64_t ldp = (w->rows + 3) & ~(int64_t)3;
         const int want = env_int("QM_LEAN_PARTS", w->units >= 32 ? 4 : 1);
@@ -966,7 +975,6 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
                 }
                 const int k = share == 2 ? (q40 ? QM_K_Q40_LEAN_X2_D4 : QM_K_Q80_LEAN_X2_D3) + di
                                          : (q40 ? QM_K_Q40_LEAN_C4D4 : QM_K_Q80_LEAN_C4D3) + (cpm == 4 ? 0 : nt == 1 ? 2 : 4) + di;
-                const bool pdl = (flags & QM_FLAG_PDL) != 0;
                 int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, pdl, false, share);
                 if (lrc || S == 1) return lrc;
                 QmSumPartsArgs sa;
@@ -1019,7 +1027,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
     const int mode = m <= 4 ? 0 : 1;
     const int k = (w->fmt == QM_FMT_Q4_0 ? QM_K_GEMV_Q40_M4 : QM_K_GEMV_Q80_M4) + mode;
     return qm_launch(c, k, (unsigned)(p.ksplit * p.ctas_per_slice), 1, (unsigned)p.consumers * 32, (unsigned)p.smem,
-                     &a, (flags & QM_FLAG_PDL) != 0);
+                     &a, pdl);
 }
 
 extern "C" int32_t qm_matvec(qm_ctx *c, qm_weight h, uint64_t x_dev, uint64_t x2_dev, int32_t m, int64_t ldx,

@@ -74,6 +74,7 @@ struct QmWeight {
     int64_t gguf_row_bytes;
     int64_t qbytes, dbytes;
     CUdeviceptr wq, wd;
+    mutable int32_t written;   // bytes were written in stream order and no launch has waited for them yet (see qm_may_overlap)
 };
 
 struct QmGemvPlan {
@@ -131,6 +132,10 @@ struct QmGemmGroup {
 int32_t qm_gemm_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
                        uint64_t c_dev, int64_t ldc, const QmGemmGroup &g);
 int qm_env_int(const char *name, int dflt);
+// Whether a launch that multiplies with w may overlap the kernel before it in the stream (programmatic stream
+// serialization). The kernels read nothing but weights before griddepcontrol.wait, so that holds for every caller once
+// the weights themselves are complete: the first launch after they were written waits for everything before it.
+bool qm_may_overlap(const QmWeight *w, uint32_t flags);
 int32_t qm_plan_fused(qm_ctx *c, int32_t m, int32_t units, bool allow_slices, QmFusedPlan *p);
 void qm_fill_op(qm_ctx *c, const QmFusedPlan &p, const QmWeight *w, uint64_t x, uint64_t x2, int64_t ldx, uint64_t y,
                 int64_t ldy, uint32_t xop, int barrier, int unit0, int units, int accumulate, QmOp *op);

@@ -767,9 +767,8 @@ extern "C" int32_t qm_ep_run(qm_ctx *c, qm_ep *e) {
     const int64_t bound = (int64_t)e->world * e->cap;   // rows this rank can receive
     int32_t rc = qm_launch(c, QM_K_EP_COLLECT, ep_grid(c, bound), 1, 256, 0, &a, false);
     if (rc) return rc;
-    // As in qm_moe_grouped, the list lengths are read back once so that the grouped launches have exactly the
-    // token tiles that hold rows; QM_MOE_NOSYNC=1 sizes them for the longest possible list instead (no
-    // synchronization; the empty CTAs cost more than the read-back on the shapes measured).
+    // The list lengths are read back once to choose the token tile; QM_MOE_NOSYNC=1 chooses it for the mean list of
+    // the largest exchange instead (no synchronization).
     int32_t longest = (int32_t)bound, typical = (int32_t)std::max<int64_t>(1, bound / e->experts);
     if (!qm_env_int("QM_MOE_NOSYNC", 0)) {
         int32_t loff[65];

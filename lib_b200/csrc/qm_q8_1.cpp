@@ -20,7 +20,7 @@ static int32_t norm_launch(qm_ctx *c, uint64_t x_dev, int64_t ldx, uint64_t weig
     a.ldx = ldx;
     a.cols = (int32_t)cols;
     a.eps = eps;
-    return qm_launch(c, QM_K_RMSNORM_Q81, (unsigned)rows, 1, 1024, 0, &a, false);
+    return qm_launch(c, QM_K_RMSNORM_Q81, (unsigned)rows, 1, 1024, 0, &a, true);
 }
 
 // The argument checks of cudaquant.RMSNormQ8_1 (quant.go:47-49) that need no data.
@@ -103,11 +103,11 @@ extern "C" int32_t qm_swiglu_q8_1(qm_ctx *c, uint64_t gate_dev, uint64_t up_dev,
     a.slots = slots;
     const int64_t blocks = ((int64_t)width * slots + 31) / 32;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((blocks + 7) / 8, (int64_t)c->sm_count * 8));
-    return qm_launch(c, QM_K_SWIGLU_Q81, grid, 1, 256, 0, &a, false);
+    return qm_launch(c, QM_K_SWIGLU_Q81, grid, 1, 256, 0, &a, true);
 }
 
 static int32_t expand_launch(qm_ctx *c, uint64_t xq_dev, int32_t m, int64_t ldx_blocks, int64_t cols, uint64_t out_dev,
-                             int64_t ld_out, bool pdl) {
+                             int64_t ld_out) {
     QmQ81ExpandArgs a;
     memset(&a, 0, sizeof a);
     a.xq = (const uint8_t *)(uintptr_t)xq_dev;
@@ -118,7 +118,7 @@ static int32_t expand_launch(qm_ctx *c, uint64_t xq_dev, int32_t m, int64_t ldx_
     a.m = m;
     const int64_t work = (int64_t)m * cols / 4;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, (int64_t)c->sm_count * 4));
-    return qm_launch(c, QM_K_Q81_EXPAND, grid, 1, 256, 0, &a, pdl);
+    return qm_launch(c, QM_K_Q81_EXPAND, grid, 1, 256, 0, &a, true);
 }
 
 extern "C" int32_t qm_q8_1_dequantize(qm_ctx *c, uint64_t xq_dev, int32_t m, int64_t ldx_blocks, int64_t cols,
@@ -129,7 +129,7 @@ extern "C" int32_t qm_q8_1_dequantize(qm_ctx *c, uint64_t xq_dev, int32_t m, int
     if (!xq_dev || !out_dev || (xq_dev & 3) || (out_dev & 15)) return QM_ERR_ARG;
     CtxGuard g(c);
     DRV(g.rc);
-    return expand_launch(c, xq_dev, m, ldx_blocks, cols, out_dev, ld_out, false);
+    return expand_launch(c, xq_dev, m, ldx_blocks, cols, out_dev, ld_out);
 }
 
 extern "C" int32_t qm_matvec_q8_1(qm_ctx *c, qm_weight h, uint64_t xq_dev, int32_t m, int64_t ldx_blocks, uint64_t y_dev,
@@ -142,14 +142,13 @@ extern "C" int32_t qm_matvec_q8_1(qm_ctx *c, qm_weight h, uint64_t xq_dev, int32
     if (!xq_dev || !y_dev || (xq_dev & 3) || (flags & 0xFu) != QM_XOP_NONE) return QM_ERR_ARG;
     CtxGuard g(c);
     DRV(g.rc);
-    const bool pdl = (flags & QM_FLAG_PDL) != 0;
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS)   // the blocks are read where they are multiplied
-        return qm_kq_launch(c, w, xq_dev, true, m, ldx_blocks, y_dev, ldy, 0, 0, 1, 0, pdl);
+        return qm_kq_launch(c, w, xq_dev, true, m, ldx_blocks, y_dev, ldy, 0, 0, 1, 0, qm_may_overlap(w, flags));
     // Q4_0 / Q8_0 / Q4_K stage and quantize their activations themselves: they get the exact float32 values
     const int64_t cols4 = (w->cols + 3) & ~(int64_t)3;
     int32_t rc = q81_scratch(c, (int64_t)m * cols4 * 4);
     if (rc) return rc;
-    rc = expand_launch(c, xq_dev, m, ldx_blocks, w->cols, c->q81_ws, cols4, pdl);
+    rc = expand_launch(c, xq_dev, m, ldx_blocks, w->cols, c->q81_ws, cols4);
     if (rc) return rc;
     return qm_matvec_launch(c, w, c->q81_ws, 0, m, cols4, y_dev, ldy, flags, c->partials_dev, c->tickets_dev);
 }
@@ -171,5 +170,5 @@ extern "C" int32_t qm_matvec_selected(qm_ctx *c, qm_weight h, int32_t experts, u
     DRV(g.rc);
     const int64_t rows_e = w->rows / experts;
     return qm_kq_launch(c, w, x_dev, xq, 1, xq ? w->cols / 32 : w->cols, y_dev, rows_e, ids_dev, experts, slots,
-                        x_slot_stride, (flags & QM_FLAG_PDL) != 0);
+                        x_slot_stride, qm_may_overlap(w, flags));
 }

@@ -40,11 +40,18 @@ __device__ __forceinline__ void store_block(uint8_t *dst, uint32_t head, int q, 
     else if (lane <= 8) reinterpret_cast<uint32_t *>(dst)[lane] = word;
 }
 
+// The launches overlap the end of the kernel before them in the stream; nothing is read or written before this.
+__device__ __forceinline__ void wait_for_inputs() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 }  // namespace
 
 // One CTA of 1024 threads per row: thread t owns elements 4t..4t+3 of every 4096-column chunk, so a block of 32
 // elements lies in eight neighbouring lanes and a row of up to 4096 columns is read from memory once.
 extern "C" __global__ void __launch_bounds__(1024) qm_rmsnorm_q8_1(const __grid_constant__ QmNormQ81Args a) {
+    wait_for_inputs();
     __shared__ double part[32];
     __shared__ int bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -121,6 +128,7 @@ extern "C" __global__ void __launch_bounds__(1024) qm_rmsnorm_q8_1(const __grid_
 }
 
 extern "C" __global__ void __launch_bounds__(256) qm_swiglu_q8_1(const __grid_constant__ QmSwigluQ81Args a) {
+    wait_for_inputs();
     const int lane = threadIdx.x & 31;
     const int64_t total = (int64_t)a.width * a.slots, blocks = (total + 31) / 32;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -158,6 +166,7 @@ extern "C" __global__ void __launch_bounds__(256) qm_swiglu_q8_1(const __grid_co
 
 // out[j][i] = widened d * q of row j's Q8_1 vector (rows ldx blocks apart; out rows ld_out floats apart).
 extern "C" __global__ void __launch_bounds__(256) qm_q8_1_expand(const __grid_constant__ QmQ81ExpandArgs a) {
+    wait_for_inputs();
     const int64_t per_row = a.cols / 4;
     const int64_t total = per_row * a.m;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {

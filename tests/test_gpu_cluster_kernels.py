@@ -75,3 +75,34 @@ def test_q8_1_row(ctx, devbuf, fmt, cols):
     assert np.abs(got[[0, 2]] - want[[0, 2]]).max() <= 2e-5 * np.abs(want[[0, 2]]).max()
     assert np.all(got[1].view(np.uint32) == 0x7fffffff)
     w.free()
+
+
+# Launches overlap the end of the kernel before them: weights written in stream order right before a product, and a
+# product whose input the launch before it writes, have to be as good as with a wait in between (equal bits).
+@pytest.mark.parametrize("fmt", [2, 8, 10, 12, 16])
+@pytest.mark.parametrize("m", [1, 8])
+def test_overlapping_launches_keep_stream_order(ctx, devbuf, fmt, m):
+    n = 1024
+    raws = [devbuf(np.frombuffer(bytes(synth.weights(fmt, n, n, seed=60 + i)), dtype=np.uint8)) for i in range(2)]
+    size = len(bytes(synth.weights(fmt, n, n, seed=60)))
+    x = devbuf(synth.activations(m, n, 5))
+
+    def chain(wait):
+        w = ctx.store_create(fmt, n, n)
+        ys = [devbuf(np.zeros((m, n), np.float32)) for _ in range(8)]
+        for i, y in enumerate(ys):
+            if i % 3 != 2:   # written before two of three products
+                w.write_rows_device(0, n, raws[i % 2].ptr, size)
+                if wait:
+                    ctx.sync()
+            ctx.matvec(w, (ys[i - 1] if i else x).ptr, m, n, y.ptr, n)
+            if wait:
+                ctx.sync()
+        ctx.sync()
+        got = [y.get((m, n)) for y in ys]
+        w.free()
+        return got
+
+    for a, b in zip(chain(True), chain(False)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    assert ctx.last_status() == (0, 0)
