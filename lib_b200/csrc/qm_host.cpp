@@ -1115,7 +1115,7 @@ static int32_t pair_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t
         p = {2, std::max(32, ((mt + nt - 1) / nt + 31) & ~31), 1};
         // few experts per GPU (expert-parallel runs) leave pairs idle: two of them share a tile's K
         // (decided by the mean list, which is known also where the lists stay on the device)
-        const int64_t most = (out_cols + 255) / 256 * ((rows_total / g.experts + 159) / 160) * g.experts;
+        const int64_t most = (out_cols + 255) / 256 * (((rows_total + g.experts - 1) / g.experts + 159) / 160) * g.experts;
         if (!g.swiglu && most <= c->gemm_clusters[1][2] && w->units >= 2 && env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0) p.splitk = 2;
     } else {
         p = plan_pair(c, out_cols, m, w->units);

@@ -106,3 +106,11 @@ def test_overlapping_launches_keep_stream_order(ctx, devbuf, fmt, m):
     for a, b in zip(chain(True), chain(False)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     assert ctx.last_status() == (0, 0)
+
+
+# More experts than rows: most lists are empty, and the down launch keeps a pair per tile (its K is shared between
+# pairs only where all tiles fit at once).
+@pytest.mark.parametrize("experts,tokens,topk", [(64, 5, 1), (64, 43, 1), (16, 9, 2), (3, 1, 2)])
+def test_moe_layer_with_few_rows(ctx, devbuf, experts, tokens, topk):
+    from tests.test_gpu_moe import TOL, run_moe
+    assert run_moe(ctx, devbuf, experts, 512, 768, tokens, topk, 23, list(range(tokens))) <= TOL
