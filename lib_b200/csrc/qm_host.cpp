@@ -1079,7 +1079,7 @@ struct QmPairPlan {
 };
 
 // Estimated cycles: a stage of 128 columns takes 4 cycles per token column on the tensor cores (a CTA alone also copies
-// and reads all of B: 6), at least what its dequantization and hand-over take; a tile's accumulator read-out is hidden
+// and reads all of B: 5), at least what its dequantization and hand-over take; a tile's accumulator read-out is hidden
 // by the next tile only where two accumulators fit.
 static QmPairPlan plan_pair(const qm_ctx *c, int64_t rows, int64_t m, int units) {
     QmPairPlan best = {2, 64, 1};

@@ -198,7 +198,7 @@ struct QmPairArgs {
     int32_t box_rows;      // token rows per tile load; a CTA's share of bn is a multiple of it
     int32_t row_tiles;     // tiles of 128 rows per CTA (SwiGLU: 64 gate rows and their up rows)
     int32_t items;         // single matmul: tiles (row tile fastest)
-    int32_t splitk;        // pairs of a cluster that share a tile's K range: 1, 2 or 4; above 1 one tile per cluster
+    int32_t splitk;        // pairs (single CTAs) of a cluster that share a tile's K range, at most four CTAs; above 1 one tile per cluster
     // Grouped launch: tokens are the rows [offsets[e], offsets[e+1]) of one matrix, the weights of expert e start at
     // wq_list[e]; an expert without rows has no tiles.
     int32_t grouped, experts;
