@@ -435,7 +435,7 @@ static int32_t upload_ops(qm_ctx *c, qm_stack *s, int m, std::vector<QmOp> &ops)
 // The op list of a step for the data-driven kernels (qm_fused_q4k_dd_*): every output buffer is
 // filled with the "not yet written" pattern before the launch and consumers poll the words they
 // read, so no grid barrier separates dependent matvecs. Needs whole tiles per CTA, no K slices
-// and one row tile of mma columns; used below the batch from which activation images win.
+// and at most two tiles of mma columns (eight rows).
 // The o and down projections are cut into K parts (QmOp::parts): their CTAs stage a quarter of x
 // each and spread over four times as many (tile, part) pieces; the consumer adds the parts up
 // while it stages them. QM_ERR_SHAPE when the step does not qualify (the caller then builds the
