@@ -233,9 +233,10 @@ struct QmListArgs {
 struct QmGatherArgs {
     const uint16_t *x;     // bf16 [tokens][ldx]
     const int32_t *list;
+    const int32_t *listed; // entries of list that hold a pair (a pair that names no expert is in no list)
     uint16_t *out;         // bf16 [rows][hidden]
     int64_t ldx;
-    int32_t rows, hidden, topk, pad;
+    int32_t rows, hidden, topk, pad;   // rows: at least *listed
 };
 struct QmCombineArgs {
     const float *y;        // [rows][hidden] expert outputs in grouped order

@@ -77,8 +77,8 @@ static inline int64_t up256(int64_t v) { return (v + 255) & ~(int64_t)255; }
 // Groups the (token, slot) pairs by expert and copies the bf16 rows of their tokens into that
 // order. Blocks until the list lengths are on the host: the caller sizes its launches (and, in
 // expert-parallel runs, its exchange) with them.
-// counts_host == nullptr: nothing is read back (no synchronization); the gather then covers all
-// pairs and *offsets_dev_out names the device array [experts + 1] of list starts.
+// counts_host == nullptr: nothing is read back (no synchronization); the gather's launch is then sized
+// for all pairs and *offsets_dev_out names the device array [experts + 1] of list starts.
 static int32_t dispatch_impl(qm_ctx *c, uint64_t ids_dev, int32_t tokens, int32_t topk, int32_t experts,
                              uint64_t x_bf16_dev, int64_t ldx, int32_t hidden, uint64_t rows_dev, uint64_t pos_dev,
                              int32_t *counts_host, CUdeviceptr *offsets_dev_out, CUdeviceptr *list_dev_out = nullptr) {
@@ -113,7 +113,7 @@ static int32_t dispatch_impl(qm_ctx *c, uint64_t ids_dev, int32_t tokens, int32_
     if (rc) return rc;
     if (offsets_dev_out) *offsets_dev_out = ws + o_offsets;
     if (list_dev_out) *list_dev_out = ws + o_list;
-    int rows = (int)pairs;   // every pair names an expert, so the lists hold all pairs
+    int rows = (int)pairs;   // at most: the gather stops at the end of the lists, which it reads on the device
     if (counts_host) {
         int32_t offsets[QM_MAX_EXPERTS + 1];
         DRV(c->drv->cuMemcpyDtoHAsync_v2(offsets, ws + o_offsets, (size_t)(experts + 1) * 4, c->stream));
@@ -128,6 +128,7 @@ static int32_t dispatch_impl(qm_ctx *c, uint64_t ids_dev, int32_t tokens, int32_
     memset(&ga, 0, sizeof ga);
     ga.x = (const uint16_t *)(uintptr_t)x_bf16_dev;
     ga.list = (const int32_t *)(uintptr_t)(ws + o_list);
+    ga.listed = la.offsets + experts;
     ga.out = (uint16_t *)(uintptr_t)rows_dev;
     ga.ldx = ldx;
     ga.rows = rows;

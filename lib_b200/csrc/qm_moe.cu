@@ -100,10 +100,11 @@ extern "C" __global__ void __launch_bounds__(1024) qm_moe_lists(const __grid_con
     }
 }
 
-// gathered[p][:] = x[token(list[p])][:], bf16 rows of `hidden` elements (16-byte pieces).
+// gathered[p][:] = x[token(list[p])][:], bf16 rows of `hidden` elements (16-byte pieces). The list ends where the pairs
+// that name an expert end: its entries beyond that were never written.
 extern "C" __global__ void __launch_bounds__(256) qm_moe_gather(const __grid_constant__ QmGatherArgs a) {
     const int pieces = a.hidden / 8;
-    const int64_t total = (int64_t)a.rows * pieces;
+    const int64_t total = (int64_t)min(a.rows, *a.listed) * pieces;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(i / pieces), c = (int)(i - (int64_t)p * pieces);
         const int pr = a.list[p];

@@ -175,6 +175,44 @@ def test_grouped_down_matmul_with_split_k(ctx, devbuf, monkeypatch):
         w.free()
 
 
+@pytest.mark.parametrize("masked", ["some", "all"])
+def test_pairs_that_name_no_expert(ctx, devbuf, monkeypatch, masked):
+    """Ids outside [0, experts) — a slot here and there, every slot of a token, the whole batch — put their pairs into no
+    list: they add nothing to the token. On a call that follows a larger one, whose longer list is still in the scratch."""
+    experts, hidden, ffn, tokens, topk, seed = 4, 512, 768, 70, 2, 57
+    run_moe(ctx, devbuf, experts, hidden, ffn, 400, topk, seed, [0])
+    gu_raw = [synth.weights(12, 2 * ffn, hidden, seed + e) for e in range(experts)]
+    dn_raw = [synth.weights(12, hidden, ffn, seed + 100 + e) for e in range(experts)]
+    gu = [ctx.store_upload(12, 2 * ffn, hidden, r) for r in gu_raw]
+    dn = [ctx.store_upload(12, hidden, ffn, r) for r in dn_raw]
+    x_bf = to_bf16_bits(synth.activations(tokens, hidden, seed + 200))
+    lg = synth.activations(tokens, experts, seed + 201)
+    ids, wts, _, wts_d = route_gpu(ctx, devbuf, lg, experts, topk)
+    if masked == "all":
+        ids[:] = -1
+    ids[3::7, 1] = -1
+    ids[5::9, 0] = experts
+    ids[[0, 44, tokens - 1]] = [[-1, experts + 7]] * 3
+    ids_d, xd = devbuf(ids), devbuf(x_bf)
+    outs = {}
+    for nosync in (None, "0"):
+        if nosync:
+            monkeypatch.setenv("QM_MOE_NOSYNC", nosync)
+        od = devbuf(np.full((tokens, hidden), np.nan, np.float32))
+        ctx.moe_grouped(gu, dn, xd.ptr, tokens, hidden, ids_d.ptr, wts_d.ptr, topk, od.ptr, hidden)
+        ctx.sync()
+        assert ctx.last_status() == (0, 0)
+        outs[nosync] = od.get((tokens, hidden))
+    gone = (ids < 0) | (ids >= experts)
+    want = moe_oracle(gu_raw, dn_raw, hidden, ffn, x_bf, np.where(gone, 0, ids), np.where(gone, np.float32(0), wts),
+                      list(range(tokens)))
+    for out in outs.values():
+        assert np.all(out[gone.all(axis=1)] == 0)
+        assert float(np.linalg.norm(out - want)) <= TOL * float(np.linalg.norm(want))
+    for w in gu + dn:
+        w.free()
+
+
 def test_layer_stages_match_oracle(ctx):
     """lib_b200.moe.MoELayer on one GPU (route -> dispatch -> experts -> combine through the
     staged entry points) against the oracle chain."""
