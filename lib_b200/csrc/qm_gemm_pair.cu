@@ -261,7 +261,7 @@ __device__ __forceinline__ void pair_body(const QmPairArgs &a) {
             uint32_t ph = 1;   // parity of the release before the stage's first use: passes at once
             bool ok = true;
             while (ok && t.next(a, offsets, stride)) {
-                const int half = ((t.mv + 15) & ~15) / CG, box = a.box_rows, nrows = (half + box - 1) / box * box;
+                const int half = qm_pair_mma_n(t.mv, CG) / CG, box = a.box_rows, nrows = (half + box - 1) / box * box;
                 const int y = t.row_off + t.m0 + rank * half;
                 for (int kc = 0; kc < nu * 2; kc++) {
                     if (!mbar_wait_bounded(empty + 8 * s, ph)) { fail(); ok = false; break; }
@@ -309,8 +309,8 @@ __device__ __forceinline__ void pair_body(const QmPairArgs &a) {
             uint32_t ph = 0, acc_ph = 1;
             bool ok = true;
             while (ok && t.next(a, offsets, stride)) {
-                // N = tokens rounded up to 16
-                const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, idesc0 | ((uint32_t)((t.mv + 15) >> 4) << 18), 0);
+                // N: bits 17..22 hold N / 8
+                const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, idesc0 | ((uint32_t)qm_pair_mma_n(t.mv, CG) << 14), 0);
                 const uint32_t d_tmem = d_tmem0 + (uint32_t)(acc * a.bn);
                 if (!warp_wait(acc_empty + 8 * acc, acc_ph)) { if (lane == 0) fail(); break; }
                 for (int kc = 0; kc < nu * 2; kc++) {

@@ -181,6 +181,18 @@ struct QmGemmArgs {
     alignas(64) CUtensorMap tmap_gather;   // the tokens' matrix, box 64 columns x 1 row, 128-byte swizzle
 };
 
+// Width N of the matrix instructions of qm_gemm_pair.cu for a tile of `tokens` tokens: with A in tensor memory and 128
+// rows per CTA the documented widths are the multiples of 16 up to 256 for one CTA and the multiples of 32 for a pair
+// (whose halves of B are N / 2 tokens; CUTLASS asserts the same in SM100_MMA_F16BF16_TS and SM100_MMA_F16BF16_2x1SM_TS).
+// A tile holds at most bn tokens, a multiple of 32, so the rounded width fits.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int qm_pair_mma_n(int tokens, int ctas) {
+    const int step = 16 * ctas;
+    return (tokens + step - 1) / step * step;
+}
+
 // Matmul by CTA pairs (qm_gemm_pair.cu): 256 weight rows x bn tokens per tile, dequantized weights in tensor memory.
 struct QmPairArgs {
     alignas(64) CUtensorMap tmap_act;  // activations [tokens][k] bf16, box 64 x box_rows, 128-byte swizzle
