@@ -62,9 +62,8 @@ extern "C" {
                                  RMSNorm+GEMV (nvidia/x/egraph/codegen.go:395-414), no gain    */
 #define QM_XOP_ADD_RMSNORM 2u /* rmsnorm(x + x2)                                               */
 #define QM_XOP_SWIGLU 3u      /* silu(x) * x2 (nvidia/x/egraph/codegen.go:328-374)             */
-#define QM_FLAG_PDL 0x100u    /* overlap the kernel before in the stream (programmatic stream serialization)
-                                 even right after the weights were written; without it the first
-                                 launch after a write waits, all others overlap                */
+#define QM_FLAG_PDL 0x100u    /* overlap the kernel before in the stream (programmatic stream
+                                 serialization); every matvec launch does, with or without it  */
 #define QM_FLAG_X_Q8_1 0x200u /* qm_matvec_selected: x holds Q8_1 blocks, not float32          */
 
 typedef struct qm_ctx qm_ctx;

@@ -480,7 +480,6 @@ extern "C" int32_t qm_store_create(qm_ctx *c, int32_t fmt, int64_t rows, int64_t
     if (fmt == QM_FMT_Q4_0) { qbytes = rows * w->units * 8 * 16; dbytes = rows * w->units * 8 * 2; }
     if (fmt == QM_FMT_Q8_0) { qbytes = rows * w->units * 8 * 32; dbytes = rows * w->units * 8 * 2; }
     w->qbytes = qbytes;
-    w->written = 1;   // the padding is zeroed in stream order
     w->dbytes = dbytes;
     CtxGuard g(c);
     CUresult r = g.rc;
@@ -501,12 +500,7 @@ extern "C" int32_t qm_store_create(qm_ctx *c, int32_t fmt, int64_t rows, int64_t
     return QM_OK;
 }
 
-bool qm_may_overlap(const QmWeight *w, uint32_t flags) {
-    return __atomic_exchange_n(&w->written, 0, __ATOMIC_RELAXED) == 0 || (flags & QM_FLAG_PDL) != 0;
-}
-
 static int32_t store_write_dev(qm_ctx *c, QmWeight *w, int64_t row_offset, int64_t nrows, CUdeviceptr src) {
-    __atomic_store_n(&w->written, 1, __ATOMIC_RELAXED);
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS) {
         DRV(c->drv->cuMemcpyDtoDAsync_v2(w->wq + row_offset * w->gguf_row_bytes, src,
                                          (size_t)(nrows * w->gguf_row_bytes), c->stream));
@@ -523,7 +517,13 @@ static int32_t store_write_dev(qm_ctx *c, QmWeight *w, int64_t row_offset, int64
     const int64_t nblk = nrows * (w->cols / (w->fmt == QM_FMT_Q4_K ? 256 : 32));
     const unsigned grid = (unsigned)std::min<int64_t>((nblk + 255) / 256, 148 * 16);
     const int k = w->fmt == QM_FMT_Q4_0 ? QM_K_REPACK_Q40 : w->fmt == QM_FMT_Q8_0 ? QM_K_REPACK_Q80 : QM_K_REPACK_Q4K;
-    return qm_launch(c, k, grid, 1, 256, 0, &a, false);
+    int32_t rc = qm_launch(c, k, grid, 1, 256, 0, &a, false);
+    if (rc) return rc;
+    // Matvecs overlap the kernel before them in the stream and read weights before they wait for it: this one-word
+    // memset, which waits for the repack like any ordinary launch, keeps the repack from being that kernel. (A mark on
+    // the weight cannot tell which stream a matvec has waited in, nor whether a captured one has run.)
+    DRV(c->drv->cuMemsetD32Async(c->gridbar_dev + 128, 0, 1, c->stream));
+    return QM_OK;
 }
 
 extern "C" int32_t qm_store_write_rows_device(qm_ctx *c, qm_weight h, int64_t row_offset, int64_t nrows,
@@ -830,25 +830,24 @@ static int32_t fused_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev,
     a.debug_slot = env_int("QM_DEBUG_OP", 0);
 #endif
     a.wait_cycles = qm_wait_cycles();
-    const bool overlap = qm_may_overlap(w, flags);
     // One op of up to four activation rows whose K fits whole: the lean body of the data-driven
     // kernels (an op that reads the launch's input polls nothing).
     if (p.slices == 1 && p.nt == 1 && p.consumers == 16 && p.depth >= 2 && p.depth <= 4 && env_int("QM_DD", 1) != 0) {
         const int k = (p.cpm == 4 ? QM_K_FUSED_Q4K_DD_C4D2 : QM_K_FUSED_Q4K_DD_C2D2) + (p.depth - 2);
         return qm_launch_ex(c, k, (unsigned)qm_fused_grid(c), (unsigned)p.consumers * 32, (unsigned)p.smem, &a,
-                            overlap, false);
+                            true, false);
     }
     const bool coop = p.slices > 1;  // K slices meet at a grid barrier: all CTAs must be co-resident
     if (coop) DRV(c->drv->cuMemsetD32Async(c->gridbar_dev, 0, 1, c->stream));
     return qm_launch_ex(c, p.nt == 1 ? QM_K_FUSED_Q4K_NT1 : QM_K_FUSED_Q4K_NT2,
                         (unsigned)qm_fused_grid(c), (unsigned)p.consumers * 32, (unsigned)p.smem, &a,
-                        overlap && !coop, coop);
+                        !coop, coop);
 }
 
 // Q2_K / IQ2_XXS: warp-per-row kernels over the GGUF bytes. x: float32 or (xq) Q8_1 blocks; ids_dev != 0: the
 // selected form over `experts` matrices stacked by rows in w, one grid row per slot, y = [slot][rows of one expert].
 int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int32_t m, int64_t ldx, uint64_t y_dev,
-                     int64_t ldy, uint64_t ids_dev, int32_t experts, int32_t slots, int64_t x_slot_stride, bool pdl) {
+                     int64_t ldy, uint64_t ids_dev, int32_t experts, int32_t slots, int64_t x_slot_stride) {
     QmKqArgs ka;
     memset(&ka, 0, sizeof ka);
     ka.wq = (const uint8_t *)(uintptr_t)w->wq;
@@ -888,7 +887,7 @@ int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int3
     const int64_t want = (ka.rows + 7) / 8;
     const int64_t cap = std::max<int64_t>(1, (int64_t)c->sm_count * per_sm / std::max(1, slots));
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, cap));
-    return qm_launch(c, k, grid, (unsigned)std::max(1, slots), 256, smem, &ka, pdl);
+    return qm_launch(c, k, grid, (unsigned)std::max(1, slots), 256, smem, &ka, true);
 }
 
 int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t x2_dev, int32_t m, int64_t ldx,
@@ -904,7 +903,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS) {
         // warp-per-row kernels over the GGUF bytes; plain products only (no fused input transform)
         if (xop != QM_XOP_NONE) return QM_ERR_ARG;
-        return qm_kq_launch(c, w, x_dev, false, m, ldx, y_dev, ldy, 0, 0, 1, 0, qm_may_overlap(w, flags));
+        return qm_kq_launch(c, w, x_dev, false, m, ldx, y_dev, ldy, 0, 0, 1, 0);
     }
     if (w->fmt == QM_FMT_Q4_K) {
         // integer tensor-core path; K is cut into slices when the activation planes of the
@@ -914,7 +913,6 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
         if (frc) return frc;
         return fused_matvec_launch(c, w, x_dev, x2_dev, m, ldx, y_dev, ldy, flags, fp);
     }
-    const bool pdl = qm_may_overlap(w, flags);
     if (env_int("QM_LEAN", 1) != 0) {
         // The integer tensor-core body: one persistent CTA of 16 warps per SM, whole tiles per CTA, per-warp
         // cp.async rings. A long K is cut into parts (CTA groups that each stage only their range of x and
@@ -975,7 +973,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
                 }
                 const int k = share == 2 ? (q40 ? QM_K_Q40_LEAN_X2_D4 : QM_K_Q80_LEAN_X2_D3) + di
                                          : (q40 ? QM_K_Q40_LEAN_C4D4 : QM_K_Q80_LEAN_C4D3) + (cpm == 4 ? 0 : nt == 1 ? 2 : 4) + di;
-                int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, pdl, false, share);
+                int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, true, false, share);
                 if (lrc || S == 1) return lrc;
                 QmSumPartsArgs sa;
                 memset(&sa, 0, sizeof sa);
@@ -1027,7 +1025,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
     const int mode = m <= 4 ? 0 : 1;
     const int k = (w->fmt == QM_FMT_Q4_0 ? QM_K_GEMV_Q40_M4 : QM_K_GEMV_Q80_M4) + mode;
     return qm_launch(c, k, (unsigned)(p.ksplit * p.ctas_per_slice), 1, (unsigned)p.consumers * 32, (unsigned)p.smem,
-                     &a, pdl);
+                     &a, true);
 }
 
 extern "C" int32_t qm_matvec(qm_ctx *c, qm_weight h, uint64_t x_dev, uint64_t x2_dev, int32_t m, int64_t ldx,

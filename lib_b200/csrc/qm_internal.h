@@ -74,7 +74,6 @@ struct QmWeight {
     int64_t gguf_row_bytes;
     int64_t qbytes, dbytes;
     CUdeviceptr wq, wd;
-    mutable int32_t written;   // bytes were written in stream order and no launch has waited for them yet (see qm_may_overlap)
 };
 
 struct QmGemvPlan {
@@ -132,17 +131,16 @@ struct QmGemmGroup {
 int32_t qm_gemm_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
                        uint64_t c_dev, int64_t ldc, const QmGemmGroup &g);
 int qm_env_int(const char *name, int dflt);
-// Whether a launch that multiplies with w may overlap the kernel before it in the stream (programmatic stream
-// serialization). The kernels read nothing but weights before griddepcontrol.wait, so that holds for every caller once
-// the weights themselves are complete: the first launch after they were written waits for everything before it.
-bool qm_may_overlap(const QmWeight *w, uint32_t flags);
 int32_t qm_plan_fused(qm_ctx *c, int32_t m, int32_t units, bool allow_slices, QmFusedPlan *p);
 void qm_fill_op(qm_ctx *c, const QmFusedPlan &p, const QmWeight *w, uint64_t x, uint64_t x2, int64_t ldx, uint64_t y,
                 int64_t ldy, uint32_t xop, int barrier, int unit0, int units, int accumulate, QmOp *op);
 int32_t qm_plan_gemv(qm_ctx *c, const QmWeight *w, int32_t m, QmGemvPlan *p);
 // The same plan for a device with `sm_count` SMs (no context needed).
 int32_t qm_plan_gemv_sms(int sm_count, const QmWeight *w, int32_t m, QmGemvPlan *p);
+// Matvec launches overlap the end of the kernel before them in the stream (programmatic stream serialization): before
+// griddepcontrol.wait they read nothing but weights, and no kernel that writes weights is ever the one before them
+// (store_write_dev).
 int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t x2_dev, int32_t m, int64_t ldx,
                          uint64_t y_dev, int64_t ldy, uint32_t flags, CUdeviceptr partials, CUdeviceptr tickets);
 int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int32_t m, int64_t ldx, uint64_t y_dev,
-                     int64_t ldy, uint64_t ids_dev, int32_t experts, int32_t slots, int64_t x_slot_stride, bool pdl);
+                     int64_t ldy, uint64_t ids_dev, int32_t experts, int32_t slots, int64_t x_slot_stride);

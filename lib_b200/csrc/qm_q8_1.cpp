@@ -143,7 +143,7 @@ extern "C" int32_t qm_matvec_q8_1(qm_ctx *c, qm_weight h, uint64_t xq_dev, int32
     CtxGuard g(c);
     DRV(g.rc);
     if (w->fmt == QM_FMT_Q2_K || w->fmt == QM_FMT_IQ2_XXS)   // the blocks are read where they are multiplied
-        return qm_kq_launch(c, w, xq_dev, true, m, ldx_blocks, y_dev, ldy, 0, 0, 1, 0, qm_may_overlap(w, flags));
+        return qm_kq_launch(c, w, xq_dev, true, m, ldx_blocks, y_dev, ldy, 0, 0, 1, 0);
     // Q4_0 / Q8_0 / Q4_K stage and quantize their activations themselves: they get the exact float32 values
     const int64_t cols4 = (w->cols + 3) & ~(int64_t)3;
     int32_t rc = q81_scratch(c, (int64_t)m * cols4 * 4);
@@ -170,5 +170,5 @@ extern "C" int32_t qm_matvec_selected(qm_ctx *c, qm_weight h, int32_t experts, u
     DRV(g.rc);
     const int64_t rows_e = w->rows / experts;
     return qm_kq_launch(c, w, x_dev, xq, 1, xq ? w->cols / 32 : w->cols, y_dev, rows_e, ids_dev, experts, slots,
-                        x_slot_stride, qm_may_overlap(w, flags));
+                        x_slot_stride);
 }

@@ -8,6 +8,7 @@ import lib_b200
 from lib_b200 import _capi, synth
 from oracle import oracle
 from tests import q8_1_cases as cases
+from tests.capture import launches
 from tests.test_gpu_matmul import TOL as MATMUL_TOL, run as run_matmul
 from tests.test_gpu_stack import build_stack, nre, oracle_chain
 
@@ -106,6 +107,35 @@ def test_overlapping_launches_keep_stream_order(ctx, devbuf, fmt, m):
     for a, b in zip(chain(True), chain(False)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     assert ctx.last_status() == (0, 0)
+
+
+# A product reads its weights before it waits for the kernel before it, so that kernel must not be the one that writes
+# them: whatever another context, on another stream, has multiplied with them in the meantime.
+@pytest.mark.parametrize("fmt", [2, 8, 12])
+@pytest.mark.parametrize("flags", [0, _capi.FLAG_PDL])
+def test_no_product_overlaps_the_kernel_that_writes_its_weights(ctx, devbuf, fmt, flags):
+    n = 1024
+    raw = devbuf(np.frombuffer(bytes(synth.weights(fmt, n, n, seed=70)), dtype=np.uint8))
+    x, y, z = devbuf(synth.activations(1, n, 5)), devbuf(nbytes=4 * n), devbuf(nbytes=4 * n)
+    w = ctx.store_create(fmt, n, n)
+    w.write_rows_device(0, n, raw.ptr, raw.nbytes)
+    ctx.sync()
+    other = lib_b200.Context(0)
+
+    def chain():
+        w.write_rows_device(0, n, raw.ptr, raw.nbytes)
+        other.matvec(w, x.ptr, 1, n, z.ptr, n)      # at once, on a stream of its own
+        ctx.matvec(w, x.ptr, 1, n, y.ptr, n, flags)
+        ctx.matvec(w, y.ptr, 1, n, z.ptr, n, flags)
+
+    made = launches(ctx, chain)
+    other.sync()
+    assert made[0].name.startswith("qm_repack")
+    products = [k for k in made if "gemv" in k.name or "fused" in k.name]
+    assert len(products) == 2 and products[0].overlaps is None and products[1].overlaps is not None
+    assert all("repack" not in (k.overlaps or "") for k in made)
+    other.close()
+    w.free()
 
 
 # More experts than rows: most lists are empty, and the down launch keeps a pair per tile (its K is shared between
