@@ -935,13 +935,16 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
         for (int oi = 0; oi < 3; oi++) {
             const int S = order[oi];
             if (S < 1 || w->units % S != 0) continue;
-            const int share = may_share && S == 1 && qm_fused_grid(c) % 2 == 0 ? 2 : 1, grid = qm_fused_grid(c);
+            const int grid = qm_fused_grid(c);
             if (grid % S != 0) continue;
             if (S > 1 && (!partials || 256 + (int64_t)S * m * ldp * 4 > QM_PARTIALS_BYTES)) continue;
             const int ups = w->units / S;
-            const int64_t fixed = (int64_t)planes * (ups * 256 + 64) + (int64_t)ups * nt * 160 + 512 * share + 16 * 2 * m * 64 + 128;
-            for (int di = 0; di < 2; di++) {
-                const int64_t smem = fixed + (int64_t)16 * depths[di] * stage;
+            // (shared with the two ring depths, then alone: eight Q8_0 rows of 17 units fit only alone)
+            const int forms = may_share && S == 1 && grid % 2 == 0 ? 4 : 2;
+            for (int f = 0; f < forms; f++) {
+                const int share = f < forms - 2 ? 2 : 1, di = f & 1;
+                const int64_t smem = (int64_t)planes * (ups * 256 + 64) + (int64_t)ups * nt * 160 + 512 * share +
+                                     16 * 2 * m * 64 + 128 + (int64_t)16 * depths[di] * stage;
                 if (smem > QM_GEMV_SMEM_MAX) continue;
                 QmLeanArgs la;
                 memset(&la, 0, sizeof la);

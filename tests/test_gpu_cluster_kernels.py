@@ -43,6 +43,24 @@ def test_matvec_shared_staging(ctx, devbuf, fmt, m, rows, cols, xop):
     w.free()
 
 
+# Eight Q8_0 rows of 17 units: the shared memory of a CTA holds them only without the second CTA's sums of squares. Sixteen
+# units, and Q4_0, share.
+@pytest.mark.parametrize("fmt,cols,kernel", [(8, 4352, "qm_gemv_q80_lean_c2n2d2"), (8, 4128, "qm_gemv_q80_lean_c2n2d2"),
+                                             (8, 4096, "qm_gemv_q80_lean_c2n2d2_x2"), (2, 4352, "qm_gemv_q40_lean_c2n2d2_x2")])
+def test_matvec_that_fits_only_without_sharing(ctx, devbuf, fmt, cols, kernel):
+    rows, m = 80, 8
+    raw = synth.weights(fmt, rows, cols, seed=cols)
+    w = ctx.store_upload(fmt, rows, cols, raw)
+    x = synth.activations(m, cols, 9)
+    xd, yd = devbuf(x), devbuf(np.full((m, rows), np.nan, np.float32))
+    call = lambda: ctx.matvec(w, xd.ptr, m, cols, yd.ptr, rows, 1)
+    assert [k.name for k in launches(ctx, call)] == [kernel]
+    call()
+    assert nre(yd.get((m, rows)), oracle.MatVec(fmt, raw, rows, cols, oracle.RMSNorm(x))) <= 3e-4
+    assert ctx.last_status() == (0, 0)
+    w.free()
+
+
 # Hidden sizes of fewer units than the cluster has warps, an odd number of units, and a down projection that cannot be
 # cut into four parts (5 and 7 units) or can (8).
 @pytest.mark.parametrize("m", [3, 4, 6, 7, 8])
