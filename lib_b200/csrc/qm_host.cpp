@@ -1074,56 +1074,17 @@ extern "C" int32_t qm_matvec_host(qm_ctx *c, qm_weight h, const float *x_host, i
 }
 
 // ---- matmul by CTA pairs ----------------------------------------------------------------------
-// The tile of a pair launch: CTAs per tile, tokens per tile, K shares per tile (one cluster).
-struct QmPairPlan {
-    int cg, bn, splitk;
-};
-
-// Estimated cycles: a stage of 128 columns takes 4 cycles per token column on the tensor cores (a CTA alone also copies
-// and reads all of B: 5), at least what its dequantization and hand-over take; a tile's accumulator read-out is hidden
-// by the next tile only where two accumulators fit.
-static QmPairPlan plan_pair(const qm_ctx *c, int64_t rows, int64_t m, int units) {
-    QmPairPlan best = {2, 64, 1};
-    double best_cost = 0;
-    for (int cg = 1; cg <= 2; cg++)
-        for (int bn = 32; bn <= 256; bn += 32) {
-            const int64_t tiles = (rows + 128 * cg - 1) / (128 * cg) * ((m + bn - 1) / bn);
-            for (int s = 1; s * cg <= 4; s *= 2) {   // clusters of up to four CTAs (of eight only 15 fit at once)
-                const int at_once = c->gemm_clusters[cg - 1][s];
-                if (at_once < 1 || (s > 1 && (tiles > at_once || units < s))) continue;
-                const int64_t rounds = (tiles + at_once - 1) / at_once;
-                const double stage = std::max((cg == 2 ? 4.0 : 5.0) * bn, 500.0), readout = 12.0 * bn + (s > 1 ? 2000 : 0);
-                const double cost = rounds * (units * 2.0 / s * stage + 500) + (bn <= 128 ? readout : rounds * readout);
-                if (best_cost == 0 || cost < best_cost) {
-                    best = {cg, bn, s};
-                    best_cost = cost;
-                }
-            }
-        }
-    return best;
-}
-
 static int32_t pair_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t m, int64_t rows_total, int64_t lda,
                            uint64_t c_dev, int64_t ldc, const QmGemmGroup &g) {
     QmPairArgs a;
     memset(&a, 0, sizeof a);
     const bool grouped = g.experts > 0;
     const int64_t out_cols = g.swiglu ? w->rows / 2 : w->rows;
-    QmPairPlan p;
-    if (grouped) {
-        // token tiles of equal size, at most 160 (an expert's weights are dequantized once per token tile)
-        const int mt = g.m_typical > 0 ? g.m_typical : m, nt = (mt + 159) / 160;
-        p = {2, std::max(32, ((mt + nt - 1) / nt + 31) & ~31), 1};
-        // few experts per GPU (expert-parallel runs) leave pairs idle: two of them share a tile's K
-        // (decided by the mean list, which is known also where the lists stay on the device)
-        const int64_t most = (out_cols + 255) / 256 * (((rows_total + g.experts - 1) / g.experts + 159) / 160) * g.experts;
-        if (!g.swiglu && most <= c->gemm_clusters[1][2] && w->units >= 2 && env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0) p.splitk = 2;
-    } else {
-        p = plan_pair(c, out_cols, m, w->units);
-    }
+    const QmPairPlan p = grouped ? qm_plan_grouped(c->gemm_clusters, out_cols, g.swiglu, m, g.m_typical > 0 ? g.m_typical : m,
+                                                   rows_total, g.experts, w->units, env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0)
+                                 : qm_plan_matmul(c->gemm_clusters, out_cols, m, w->units);
     const int tile_rows = (g.swiglu ? 64 : 128) * p.cg;
-    const int64_t row_tiles = (out_cols + tile_rows - 1) / tile_rows;
-    const int64_t tiles = row_tiles * ((m + p.bn - 1) / p.bn) * (grouped ? g.experts : 1);
+    const int64_t row_tiles = (out_cols + tile_rows - 1) / tile_rows, tiles = p.tiles;
     if (!grouped && tiles * p.cg * p.splitk > (1 << 30)) return QM_ERR_SHAPE;
     const int stage_bytes = p.bn * 256 / p.cg;
     a.bn = p.bn;

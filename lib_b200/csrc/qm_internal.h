@@ -5,6 +5,7 @@
 #include "../../include/qmatmul.h"
 #include "qm_driver.h"
 #include "qm_kernel_args.h"
+#include "qm_pair_plan.h"
 
 #define QM_CTX_MAGIC 0x514D4358u     // "QMCX"
 #define QM_WEIGHT_MAGIC 0x514D5754u  // "QMWT"
@@ -50,7 +51,7 @@ struct qm_ctx {
     bool have_ctx;
     int sm_count, l2_bytes;
     CUmodule modules[QM_MOD_COUNT];
-    int gemm_clusters[2][5];   // [CTAs per tile - 1][K shares]: clusters of the matmul by CTA pairs that run at once
+    QmPairClusters gemm_clusters;
     int max_clusters[5];   // clusters of 2 and 4 GEMV CTAs (512 threads, all of the shared memory) that run at once
     CUfunction fn[QM_K_COUNT];
     CUstream own_stream, stream;

@@ -162,3 +162,26 @@ def test_no_product_overlaps_the_kernel_that_writes_its_weights(ctx, devbuf, fmt
 def test_moe_layer_with_few_rows(ctx, devbuf, experts, tokens, topk):
     from tests.test_gpu_moe import TOL, run_moe
     assert run_moe(ctx, devbuf, experts, 512, 768, tokens, topk, 23, list(range(tokens))) <= TOL
+
+
+# Lists far longer than the mean, which the token tile is chosen for and which the host does not know: every token to one
+# expert, K shared between pairs (four experts of hidden 512) and not (64 experts).
+@pytest.mark.parametrize("experts,tokens", [(4, 40), (4, 333), (64, 200)])
+def test_moe_layer_with_one_long_list(ctx, devbuf, experts, tokens):
+    from tests.test_gpu_moe import TOL, moe_oracle, to_bf16_bits
+    hidden, ffn, seed = 512, 768, 29
+    gu_raw = [synth.weights(12, 2 * ffn, hidden, seed + e) for e in range(experts)]
+    dn_raw = [synth.weights(12, hidden, ffn, seed + 100 + e) for e in range(experts)]
+    gu = [ctx.store_upload(12, 2 * ffn, hidden, r) for r in gu_raw]
+    dn = [ctx.store_upload(12, hidden, ffn, r) for r in dn_raw]
+    x_bf = to_bf16_bits(synth.activations(tokens, hidden, seed + 200))
+    ids, wts = np.full((tokens, 1), 2, np.int32), np.ones((tokens, 1), np.float32)
+    out_d = devbuf(np.full((tokens, hidden), np.nan, np.float32))
+    ctx.moe_grouped(gu, dn, devbuf(x_bf).ptr, tokens, hidden, devbuf(ids).ptr, devbuf(wts).ptr, 1, out_d.ptr, hidden)
+    ctx.sync()
+    assert ctx.last_status() == (0, 0)
+    want = moe_oracle(gu_raw, dn_raw, hidden, ffn, x_bf, ids, wts, list(range(tokens)))
+    got = out_d.get((tokens, hidden))
+    assert np.isfinite(got).all() and float(np.linalg.norm(got - want)) <= TOL * float(np.linalg.norm(want))
+    for w in gu + dn:
+        w.free()
