@@ -37,6 +37,7 @@
     X(cuStreamCreate, CUresult (*)(CUstream *, unsigned int))                                     \
     X(cuStreamDestroy_v2, CUresult (*)(CUstream))                                                 \
     X(cuStreamSynchronize, CUresult (*)(CUstream))                                                \
+    X(cuStreamIsCapturing, CUresult (*)(CUstream, CUstreamCaptureStatus *))                       \
     X(cuStreamBeginCapture_v2, CUresult (*)(CUstream, CUstreamCaptureMode))                       \
     X(cuStreamEndCapture, CUresult (*)(CUstream, CUgraph *))                                      \
     X(cuGraphInstantiateWithFlags, CUresult (*)(CUgraphExec *, CUgraph, unsigned long long))      \

@@ -51,6 +51,14 @@ static int32_t ensure_ws(qm_ctx *c, int64_t bytes) { return grow(c, &c->moe_ws, 
 static int32_t ensure_ws2(qm_ctx *c, int64_t bytes) { return grow(c, &c->moe_ws2, &c->moe_ws2_bytes, bytes); }
 static int32_t ensure_ws3(qm_ctx *c, int64_t bytes) { return grow(c, &c->moe_ws3, &c->moe_ws3_bytes, bytes); }
 
+// The expert stage copies its tables from this call's own frame: a captured copy would read that memory again when the
+// graph runs. Refused like the synchronization that a call with the list lengths read back makes.
+static int32_t refuse_capture(qm_ctx *c) {
+    CUstreamCaptureStatus status = CU_STREAM_CAPTURE_STATUS_NONE;
+    DRV(c->drv->cuStreamIsCapturing(c->stream, &status));
+    return status == CU_STREAM_CAPTURE_STATUS_NONE ? QM_OK : (int32_t)CUDA_ERROR_STREAM_CAPTURE_UNSUPPORTED;
+}
+
 static int32_t check_experts(const qm_weight *gate_up, const qm_weight *down, int32_t experts,
                              std::vector<QmWeight *> &wg, std::vector<QmWeight *> &wd, int64_t *hidden, int64_t *ffn) {
     if (!gate_up || !down) return QM_ERR_ARG;
@@ -214,6 +222,8 @@ extern "C" int32_t qm_moe_experts(qm_ctx *c, const qm_weight *gate_up, const qm_
     if (rows >= (1 << 24)) return QM_ERR_SHAPE;
     CtxGuard g(c);
     DRV(g.rc);
+    rc = refuse_capture(c);
+    if (rc) return rc;
     // workspace: the bf16 hidden activations, the offsets, then the two lists of weight stores
     const int64_t o_off = up256(rows * ffn * 2), total = o_off + up256((QM_MAX_EXPERTS + 1) * 4) + 2 * QM_MAX_EXPERTS * 8;
     rc = ensure_ws2(c, total);
@@ -265,7 +275,8 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
     {
         CtxGuard g(c);
         DRV(g.rc);
-        rc = ensure_ws3(c, total);
+        rc = refuse_capture(c);
+        if (!rc) rc = ensure_ws3(c, total);
         if (rc) return rc;
     }
     const CUdeviceptr ws = c->moe_ws3;

@@ -6,8 +6,10 @@ Tolerance of the grouped matmul: normwise 3e-3 (bf16 activations on the tensor c
 import numpy as np
 import pytest
 
+import lib_b200
 from lib_b200 import synth
 from oracle import oracle
+from tests.capture import launches
 
 pytestmark = pytest.mark.gpu
 TOL = 3e-3
@@ -209,6 +211,36 @@ def test_pairs_that_name_no_expert(ctx, devbuf, monkeypatch, masked):
     for out in outs.values():
         assert np.all(out[gone.all(axis=1)] == 0)
         assert float(np.linalg.norm(out - want)) <= TOL * float(np.linalg.norm(want))
+    for w in gu + dn:
+        w.free()
+
+
+def test_layer_is_not_captured(ctx, devbuf):
+    """The expert stage's tables come from the call's own frame, so a graph of it could not be replayed: refused, with
+    nothing in the graph, and the stream works as before."""
+    experts, hidden, ffn = 2, 256, 256
+    gu = [ctx.store_upload(12, 2 * ffn, hidden, synth.weights(12, 2 * ffn, hidden, e)) for e in range(experts)]
+    dn = [ctx.store_upload(12, hidden, ffn, synth.weights(12, hidden, ffn, 9 + e)) for e in range(experts)]
+    b = [devbuf(np.zeros(4096, np.uint8)) for _ in range(4)]
+
+    def layer():
+        ctx.moe_grouped(gu, dn, b[0].ptr, 2, hidden, b[1].ptr, b[2].ptr, 1, b[3].ptr, hidden)
+
+    def expert_stage():
+        ctx.moe_experts(gu, dn, b[0].ptr, [1, 1], b[3].ptr)
+
+    for call in (layer, expert_stage):
+        call()
+
+        def refused():
+            with pytest.raises(lib_b200.QmError) as e:
+                call()
+            assert e.value.code == 900      # CUDA_ERROR_STREAM_CAPTURE_UNSUPPORTED
+
+        assert launches(ctx, refused) == []
+        call()
+    ctx.sync()
+    assert ctx.last_status() == (0, 0)
     for w in gu + dn:
         w.free()
 
