@@ -43,17 +43,15 @@ def _run(cmd):
     return r.stdout
 
 
-def _describe(src, cubin, ptxas_log):
-    """Kernel table for Go callers that load the cubin through nvidia/driver."""
-    text = open(src).read()
-    names = re.findall(r'QM_(?:GEMV|DD|KQ|DD_SEL|LEAN|DD8)_KERNEL\((\w+),', text) + re.findall(
-        r'extern "C" __global__ void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\(', text)
+def _describe(cubin, ptxas_log):
+    """Kernel table for Go callers that load the cubin through nvidia/driver: every entry that ptxas reports."""
     res = {}
     cur = None
     for line in ptxas_log.splitlines():
         m = re.search(r"Compiling entry function '(\w+)'", line)
         if m:
             cur = m.group(1)
+            res[cur] = {}
         m = re.search(r"Used (\d+) registers", line)
         if m and cur:
             res[cur] = {"registers": int(m.group(1))}
@@ -61,7 +59,7 @@ def _describe(src, cubin, ptxas_log):
             "kernels": [{"entry_point": n,
                          "schema": [{"name": "args", "kind": "struct_by_value",
                                      "defined_in": "lib_b200/csrc/qm_kernel_args.h"}],
-                         "resources": res.get(n, {})} for n in names if n != "name"]}
+                         "resources": r} for n, r in res.items()]}
 
 
 def build(force=False, verbose=False):
@@ -79,7 +77,7 @@ def build(force=False, verbose=False):
             if verbose:
                 print(log)
             with open(cubin[:-6] + ".json", "w") as f:
-                json.dump(_describe(src, cubin, log), f, indent=1)
+                json.dump(_describe(cubin, log), f, indent=1)
     srcs = [os.path.join(CSRC, s) for s in HOST_SOURCES]
     # translation units that use the CUDA runtime (kernels launched with <<<>>>)
     rt_objs = []

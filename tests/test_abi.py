@@ -1,7 +1,10 @@
 """CPU tests of the drop-in boundary: the shared library loads without a GPU,
 exports every symbol include/qmatmul.h declares, and reports errors as codes."""
 import ctypes
+import glob
+import json
 import os
+import re
 
 import pytest
 
@@ -40,6 +43,18 @@ def test_kernel_images_and_descriptions_are_built():
         assert os.path.getsize(cubin) > 1000
         assert open(cubin, "rb").read(4) == b"\x7fELF"
         assert os.path.exists(os.path.join(d, stem + ".sm_100a.json"))
+
+
+def test_every_kernel_is_described():
+    root = os.path.dirname(_capi._LIB_PATH)
+    host = open(os.path.join(root, "csrc", "qm_host.cpp")).read()
+    wanted = set(re.findall(r'\{QM_MOD_\w+,\s*"(\w+)"\}', host))
+    described = set()
+    for f in glob.glob(os.path.join(root, "csrc", "build", "*.json")):
+        for k in json.load(open(f))["kernels"]:
+            described.add(k["entry_point"])
+            assert k["resources"]["registers"] > 0
+    assert len(wanted) > 50 and described == wanted
 
 
 @pytest.mark.skipif(os.path.exists("/dev/nvidiactl"), reason="only meaningful without a GPU")
