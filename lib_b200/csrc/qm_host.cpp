@@ -1081,7 +1081,9 @@ static int32_t pair_launch(qm_ctx *c, const QmWeight *w, uint64_t a_dev, int32_t
     const bool grouped = g.experts > 0;
     const int64_t out_cols = g.swiglu ? w->rows / 2 : w->rows;
     const QmPairPlan p = grouped ? qm_plan_grouped(c->gemm_clusters, out_cols, g.swiglu, m, g.m_typical > 0 ? g.m_typical : m,
-                                                   rows_total, g.experts, w->units, env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0)
+                                                   rows_total, g.experts, w->units, env_int("QM_GEMM_GROUPED_SPLITK", 1) != 0,
+                                                   g.share_longest > 0 ? g.share_longest : m,
+                                                   g.share_longest > 0 ? g.share_rows : rows_total)
                                  : qm_plan_matmul(c->gemm_clusters, out_cols, m, w->units);
     const int tile_rows = (g.swiglu ? 64 : 128) * p.cg;
     const int64_t row_tiles = (out_cols + tile_rows - 1) / tile_rows, tiles = p.tiles;

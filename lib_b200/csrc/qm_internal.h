@@ -118,7 +118,8 @@ int64_t qm_wait_cycles();
 void qm_balance_op(qm_ctx *c, QmOp *op);
 struct QmGemmGroup {
     int experts;               // 0: a single matmul
-    int m_typical;             // 0, or the list length to choose the token tile for (the grid still covers m)
+    int m_typical;             // 0, or the list length to choose the token tile for (the launch still covers m)
+    int64_t share_longest, share_rows;   // 0, or the bounds on the lists that decide whether K is shared (qm_plan_grouped)
     CUdeviceptr wq_list_dev;   // device array of the experts' weight stores
     CUdeviceptr offsets_dev;   // device array [experts + 1]: first activation row of each expert
     bool swiglu;               // gate|up weights, output bf16 silu(gate)*up to h_dev

@@ -2,7 +2,6 @@
 // matmul that reuses the quantized prefill GEMM over per-expert token lists.
 // The Go-facing surface it stands behind is lm/moe: GroupedTopKRouter.Route
 // (lm/moe/moe.go:73-141) for the routing; the grouped matmul is new API of this path.
-#include <math.h>
 #include <string.h>
 
 #include <algorithm>
@@ -154,11 +153,12 @@ extern "C" int32_t qm_moe_dispatch(qm_ctx *c, uint64_t ids_dev, int32_t tokens, 
 }
 
 // The two grouped launches over rows grouped by expert (list starts in offsets_dev): gate|up with
-// the SwiGLU in the epilogue (bf16 h in the stage's workspace), then down into y. `longest`
-// bounds the list lengths (sizes the grid), `typical` chooses the token tile.
+// the SwiGLU in the epilogue (bf16 h in the stage's workspace), then down into y. `longest` and
+// `rows` bound the lists (they bound the launches), `typical` chooses the token tile; share_pairs:
+// 0, or the pairs that decide on sharing K whether the lists are known or not.
 static int32_t experts_launch(qm_ctx *c, const std::vector<QmWeight *> &wg, const std::vector<QmWeight *> &wd,
                               int32_t experts, uint64_t rows_bf16_dev, int64_t rows, int32_t longest, int32_t typical,
-                              CUdeviceptr offsets_dev, uint64_t y_dev, int64_t hidden, int64_t ffn,
+                              CUdeviceptr offsets_dev, uint64_t y_dev, int64_t hidden, int64_t ffn, int64_t share_pairs,
                               CUdeviceptr gather_list_dev = 0, int gather_topk = 0, int64_t x_rows = 0, int64_t ldx = 0) {
     const int64_t o_h = 0, o_gl = up256(rows * ffn * 2) + up256((QM_MAX_EXPERTS + 1) * 4), o_dl = o_gl + QM_MAX_EXPERTS * 8,
                   total = o_dl + QM_MAX_EXPERTS * 8;
@@ -176,6 +176,7 @@ static int32_t experts_launch(qm_ctx *c, const std::vector<QmWeight *> &wg, cons
     memset(&grp, 0, sizeof grp);
     grp.experts = experts;
     grp.m_typical = typical;
+    grp.share_longest = grp.share_rows = share_pairs;
     grp.offsets_dev = offsets_dev;
     grp.wq_list_dev = ws + o_gl;
     grp.swiglu = true;
@@ -199,8 +200,8 @@ static int32_t experts_launch(qm_ctx *c, const std::vector<QmWeight *> &wg, cons
 // y[p][:] = down_e( silu(gate_e r_p) * (up_e r_p) ) for rows r grouped by expert: the first
 // counts[0] rows belong to expert 0, the next counts[1] to expert 1, and so on. Two launches
 // for all experts together: gate|up with the SwiGLU in the epilogue (bf16 h), then down.
-extern "C" int32_t qm_moe_experts(qm_ctx *c, const qm_weight *gate_up, const qm_weight *down, int32_t experts,
-                                  uint64_t rows_bf16_dev, const int32_t *counts_host, uint64_t y_dev) {
+static int32_t experts_impl(qm_ctx *c, const qm_weight *gate_up, const qm_weight *down, int32_t experts,
+                            uint64_t rows_bf16_dev, const int32_t *counts_host, uint64_t y_dev, int64_t share_pairs) {
     CHECK_CTX(c);
     if (!rows_bf16_dev || !counts_host || !y_dev) return QM_ERR_ARG;
     std::vector<QmWeight *> wg, wd;
@@ -231,7 +232,13 @@ extern "C" int32_t qm_moe_experts(qm_ctx *c, const qm_weight *gate_up, const qm_
     const CUdeviceptr ws = c->moe_ws2;
     // the offsets travel in stream order; the host copy is read before the call returns
     DRV(c->drv->cuMemcpyHtoDAsync_v2(ws + o_off, offsets, (size_t)(experts + 1) * 4, c->stream));
-    return experts_launch(c, wg, wd, experts, rows_bf16_dev, rows, longest, longest, ws + o_off, y_dev, hidden, ffn);
+    return experts_launch(c, wg, wd, experts, rows_bf16_dev, rows, longest, longest, ws + o_off, y_dev, hidden, ffn,
+                          share_pairs);
+}
+
+extern "C" int32_t qm_moe_experts(qm_ctx *c, const qm_weight *gate_up, const qm_weight *down, int32_t experts,
+                                  uint64_t rows_bf16_dev, const int32_t *counts_host, uint64_t y_dev) {
+    return experts_impl(c, gate_up, down, experts, rows_bf16_dev, counts_host, y_dev, 0);
 }
 
 // out[t][:] = sum_s weights[t][s] * y[pos[t*topk+s]][:], slots in order (deterministic).
@@ -311,7 +318,7 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
             CtxGuard g(c);
             DRV(g.rc);
             rc = experts_launch(c, wg, wd, experts, x_bf16_dev, pairs, longest, typical, offsets_dev, ws + o_y, hidden, ffn,
-                                list_dev, topk, tokens, ldx);
+                                pairs, list_dev, topk, tokens, ldx);
             if (rc) return rc;
         }
         return qm_moe_combine(c, ws + o_y, ws + o_pos, weights_dev, tokens, topk, (int32_t)hidden, out_dev, ldo);
@@ -321,7 +328,7 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
         rc = qm_moe_dispatch(c, ids_dev, tokens, topk, experts, x_bf16_dev, ldx, (int32_t)hidden, ws + o_rows, ws + o_pos,
                              counts);
         if (rc) return rc;
-        rc = qm_moe_experts(c, gate_up, down, experts, ws + o_rows, counts, ws + o_y);
+        rc = experts_impl(c, gate_up, down, experts, ws + o_rows, counts, ws + o_y, pairs);
         if (rc) return rc;
         return qm_moe_combine(c, ws + o_y, ws + o_pos, weights_dev, tokens, topk, (int32_t)hidden, out_dev, ldo);
     }
@@ -333,10 +340,8 @@ extern "C" int32_t qm_moe_grouped(qm_ctx *c, const qm_weight *gate_up, const qm_
         CtxGuard g(c);
         DRV(g.rc);
         if (pairs >= (1 << 24)) return QM_ERR_SHAPE;   // as qm_moe_experts
-        const double mean = (double)pairs / experts;
-        const int32_t typical = (int32_t)std::max(1.0, mean + 2.0 * sqrt(mean));
-        rc = experts_launch(c, wg, wd, experts, ws + o_rows, pairs, (int32_t)pairs, typical, offsets_dev, ws + o_y, hidden,
-                            ffn);
+        rc = experts_launch(c, wg, wd, experts, ws + o_rows, pairs, (int32_t)pairs, (int32_t)qm_typical_list(pairs, experts),
+                            offsets_dev, ws + o_y, hidden, ffn, pairs);
         if (rc) return rc;
     }
     return qm_moe_combine(c, ws + o_y, ws + o_pos, weights_dev, tokens, topk, (int32_t)hidden, out_dev, ldo);
@@ -793,7 +798,7 @@ extern "C" int32_t qm_ep_run(qm_ctx *c, qm_ep *e) {
     }
     if (longest > 0) {
         rc = experts_launch(c, e->wg, e->wd, e->eloc, e->local + e->o_compact, bound, longest, typical,
-                            e->local + e->o_loff, e->local + e->o_y, e->hidden, e->ffn);
+                            e->local + e->o_loff, e->local + e->o_y, e->hidden, e->ffn, 0);
         if (rc) return rc;
     }
     rc = qm_launch(c, QM_K_EP_RETURN, ep_grid(c, bound), 1, 256, 0, &a, false);

@@ -1,5 +1,6 @@
 // Which tile a matmul by CTA pairs (qm_gemm_pair.cu) runs with. Host code without a context: sizes in, plan out.
 #pragma once
+#include <math.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -44,19 +45,37 @@ inline int64_t qm_grouped_token_tiles(int64_t longest, int64_t rows, int64_t exp
     return std::min(experts * ((longest + bn - 1) / bn), (rows + std::min(experts, rows) * (bn - 1)) / bn);
 }
 
-// Grouped launch: `experts` matrices of out_cols output columns (with SwiGLU: gate rows) over token lists that the host
-// knows only the bounds of. Token tiles of equal size, at most 160, chosen for lists of `typical` tokens.
+// Tokens per tile for lists of l tokens: tiles of equal size, at most 160.
+inline int qm_grouped_bn(int64_t l) {
+    const int64_t nt = (l + 159) / 160;
+    return (int)std::max<int64_t>(32, ((l + nt - 1) / nt + 31) & ~(int64_t)31);
+}
+
+// The list length that a tile is chosen for where only the mean is known: two standard deviations of a random choice more.
+inline int64_t qm_typical_list(int64_t rows, int64_t experts) {
+    const double mean = (double)rows / experts;
+    return (int64_t)std::max(1.0, mean + 2.0 * sqrt(mean));
+}
+
+// Grouped launch: `experts` matrices of out_cols output columns (with SwiGLU: gate rows) over token lists of at most
+// `longest` tokens, `rows` together; tiles chosen for lists of `typical` tokens.
 // Few experts (expert-parallel runs) leave pairs idle: two of them then share a tile's K. A K-shared launch starts a
 // cluster per tile that the lists may hold, so it is taken only where all of those fit at once, and whether it may be is
 // seen from the bound on the tiles, not from a mean list. MoE layers, shared -> not: 1 expert 4096 x 4096 of 128 tokens
 // 61 -> 65 us, 2 experts 1024 x 4096 of 64 tokens 48 -> 52; where clusters stand in line for tiles that are mostly empty,
 // 16 experts 512 x 2048 of 1024 pairs 138 -> 64 us, 4 experts 2048 x 4096 of 600 pairs 115 -> 83.
+// Sharing K changes the order of additions. It is decided by share_longest and share_rows, which a caller that may know
+// the lists or not gives as the bounds that hold in both cases, so that the bits do not depend on which.
 inline QmPairPlan qm_plan_grouped(const QmPairClusters &clusters, int64_t out_cols, bool swiglu, int64_t longest,
-                                  int64_t typical, int64_t rows, int experts, int units, bool may_share) {
-    const int64_t nt = (typical + 159) / 160;
-    QmPairPlan p = {2, (int)std::max<int64_t>(32, ((typical + nt - 1) / nt + 31) & ~(int64_t)31), 1, 0};
+                                  int64_t typical, int64_t rows, int experts, int units, bool may_share,
+                                  int64_t share_longest, int64_t share_rows) {
     const int tile_rows = swiglu ? 128 : 256;
-    p.tiles = (out_cols + tile_rows - 1) / tile_rows * qm_grouped_token_tiles(longest, rows, experts, p.bn);
-    if (may_share && !swiglu && units >= 2 && p.tiles <= clusters[1][2]) p.splitk = 2;
+    const int64_t row_tiles = (out_cols + tile_rows - 1) / tile_rows;
+    QmPairPlan p = {2, qm_grouped_bn(typical), 1, 0};
+    p.tiles = row_tiles * qm_grouped_token_tiles(longest, rows, experts, p.bn);
+    const int share_bn = qm_grouped_bn(qm_typical_list(share_rows, experts));
+    if (may_share && !swiglu && units >= 2 &&
+        row_tiles * qm_grouped_token_tiles(share_longest, share_rows, experts, share_bn) <= clusters[1][2])
+        p.splitk = 2;
     return p;
 }

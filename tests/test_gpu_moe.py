@@ -177,6 +177,28 @@ def test_grouped_down_matmul_with_split_k(ctx, devbuf, monkeypatch):
         w.free()
 
 
+@pytest.mark.parametrize("experts,tokens,topk", [(16, 512, 2), (2, 150, 2), (3, 400, 1)])
+def test_bits_do_not_depend_on_where_the_lengths_are_known(ctx, devbuf, monkeypatch, experts, tokens, topk):
+    """Whether pairs of CTAs share K, which changes the order of additions, is decided alike: shapes where the tiles of the
+    lists themselves would fit at once and those that the lists may hold would not, and where both fit."""
+    hidden, ffn, seed = 512, 512, 61
+    gu = [ctx.store_upload(12, 2 * ffn, hidden, synth.weights(12, 2 * ffn, hidden, seed + e)) for e in range(experts)]
+    dn = [ctx.store_upload(12, hidden, ffn, synth.weights(12, hidden, ffn, seed + 100 + e)) for e in range(experts)]
+    xd = devbuf(to_bf16_bits(synth.activations(tokens, hidden, seed + 200)))
+    _, _, ids_d, wts_d = route_gpu(ctx, devbuf, synth.activations(tokens, experts, seed + 201), experts, topk)
+    outs = []
+    for nosync, fold in (("1", "0"), ("0", "0"), ("0", "1")):
+        monkeypatch.setenv("QM_MOE_NOSYNC", nosync)
+        monkeypatch.setenv("QM_MOE_FOLD", fold)
+        od = devbuf(np.full((tokens, hidden), np.nan, np.float32))
+        ctx.moe_grouped(gu, dn, xd.ptr, tokens, hidden, ids_d.ptr, wts_d.ptr, topk, od.ptr, hidden)
+        outs.append(od.get((tokens, hidden)).view(np.uint32))
+    assert ctx.last_status() == (0, 0)
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+    for w in gu + dn:
+        w.free()
+
+
 @pytest.mark.parametrize("masked", ["some", "all"])
 def test_pairs_that_name_no_expert(ctx, devbuf, monkeypatch, masked):
     """Ids outside [0, experts) — a slot here and there, every slot of a token, the whole batch — put their pairs into no

@@ -48,17 +48,43 @@ def test_token_tiles_of_expert_lists_are_bounded_tightly(tmp_path):
 
 
 def test_shared_k_launches_fit_at_once(tmp_path):
-    """Grouped down launches share K only where a cluster per possible tile fits on the device at once."""
-    cases = [(hidden, longest, typical, rows, experts) for hidden in (512, 1024, 2048, 4096) for experts in (1, 2, 4, 8, 16, 64)
-             for rows in (3, 64, 300, 600, 1024, 8192) for longest in (rows, (rows + experts - 1) // experts)
-             for typical in ((rows + experts - 1) // experts,)]
+    """Grouped down launches over lists that stay on the device share K only where a cluster for every tile that the lists
+    may hold fits on the device at once; where the host knows the lists of the same pairs, it decides alike."""
+    cases = [(hidden, rows, experts) for hidden in (512, 1024, 2048, 4096) for experts in (1, 2, 4, 8, 16, 64)
+             for rows in (3, 64, 300, 600, 1024, 8192)]
+    body = CLUSTERS + "\nQmPairPlan p;\n"
+    for hidden, rows, experts in cases:
+        for longest, typical in ((rows, "qm_typical_list(%d, %d)" % (rows, experts)), ((rows + experts - 1) // experts,) * 2):
+            body += ('p = qm_plan_grouped(at_once, %d, false, %d, %s, %d, %d, 16, true, %d, %d); '
+                     'printf("%%d %%d %%d %%d\\n", p.cg, p.bn, p.splitk, (int)p.tiles);\n'
+                     % (hidden, longest, typical, rows, experts, rows, rows))
+    lines = [tuple(map(int, line.split())) for line in compiled(tmp_path, body, "qm_pair_plan.h").splitlines()]
+    for case, unknown, known in zip(cases, lines[::2], lines[1::2]):
+        for cg, bn, splitk, tiles in (unknown, known):
+            assert cg == 2 and bn % 32 == 0 and 32 <= bn <= 160 and tiles >= 1
+        assert unknown[2] == (2 if unknown[3] <= 33 else 1) == known[2], case
+    assert {p[2] for p in lines} == {1, 2}
+
+
+# One shape per form of the single-matrix matmul: rows, K, tokens -> CTAs per tile, tokens per tile, K shares, tiles.
+# Ragged rows; token tiles that are full, that end one token past a multiple of 16 or 32, and short last ones.
+FORMS = [
+    ((10129, 256, 103), (2, 128, 1, 40)), ((4862, 1536, 103), (2, 128, 2, 19)), ((6144, 4096, 391), (2, 160, 1, 72)),
+    ((10129, 256, 145), (2, 160, 1, 40)), ((4862, 2816, 139), (2, 160, 2, 19)), ((12934, 512, 169), (2, 192, 1, 51)),
+    ((775, 3840, 1411), (2, 192, 2, 32)), ((12934, 768, 205), (2, 224, 1, 51)), ((4862, 9216, 205), (2, 224, 2, 19)),
+    ((1739, 2304, 1908), (2, 192, 1, 70)), ((14336, 1024, 2048), (2, 128, 1, 896)),
+    ((64, 1024, 2), (1, 32, 4, 1)), ((4302, 1536, 2), (1, 32, 2, 34)), ((536, 256, 962), (1, 64, 1, 80)),
+    ((4862, 1536, 36), (1, 64, 2, 38)), ((64, 1024, 1059), (1, 64, 4, 17)), ((10129, 256, 69), (1, 96, 1, 80)),
+    ((4862, 1536, 69), (1, 96, 2, 38)), ((137, 1024, 1059), (1, 96, 4, 24)), ((1616, 256, 1282), (1, 128, 1, 143)),
+    ((536, 2048, 1411), (1, 128, 2, 60)), ((137, 1536, 1553), (1, 128, 4, 26)), ((2638, 256, 962), (1, 160, 1, 147)),
+    ((775, 3840, 1553), (1, 160, 2, 70)), ((289, 2048, 1553), (1, 160, 4, 30)), ((6210, 2816, 490), (1, 192, 1, 147)),
+    ((6210, 768, 655), (1, 224, 1, 147)),
+]
+
+
+def test_matmul_plans(tmp_path):
     body = CLUSTERS + "\nQmPairPlan p;\n" + "\n".join(
-        'p = qm_plan_grouped(at_once, %d, false, %d, %d, %d, %d, 16, true); printf("%%d %%d %%d %%d\\n", p.cg, p.bn, p.splitk, '
-        '(int)p.tiles);' % c for c in cases)
-    shared = 0
-    for c, line in zip(cases, compiled(tmp_path, body, "qm_pair_plan.h").splitlines()):
-        cg, bn, splitk, tiles = map(int, line.split())
-        assert cg == 2 and bn % 32 == 0 and 32 <= bn <= 160 and tiles >= 1
-        assert splitk == (2 if tiles <= 33 else 1), c
-        shared += splitk == 2
-    assert 0 < shared < len(cases)
+        'p = qm_plan_matmul(at_once, %d, %d, %d); printf("%%d %%d %%d %%d\\n", p.cg, p.bn, p.splitk, (int)p.tiles);'
+        % (n, m, k // 256) for (n, k, m), _ in FORMS)
+    out = compiled(tmp_path, body, "qm_pair_plan.h")
+    assert [tuple(map(int, line.split())) for line in out.splitlines()] == [plan for _, plan in FORMS]
