@@ -525,12 +525,13 @@ QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m4, 16, 4, true)
 QM_KQ_KERNEL(qm_gemv_iq2xxs_q81_m8, 16, 8, true)
 
 // One Q8_1 row through the staged form, K up to 4096 (kernels of their own: the registers that hold the activations
-// would cost the direct form its occupancy; with one entry for both it lost up to 10 %).
-#define QM_KQ_ROW_KERNEL(name, fmt)                                                                            \
-    extern "C" __global__ void __launch_bounds__(256) name(const __grid_constant__ QmKqArgs a) {               \
+// would cost the direct form its occupancy; with one entry for both it lost up to 10 %). `ctas` of them fit on an SM by
+// registers: the host launches no more than run at once.
+#define QM_KQ_ROW_KERNEL(name, fmt, ctas)                                                                      \
+    extern "C" __global__ void __launch_bounds__(256, ctas) name(const __grid_constant__ QmKqArgs a) {         \
         __shared__ uint32_t tab[fmt == 16 ? 384 * kCopies : 1];                                                \
         if (a.units <= 8) gemv_kq_q81_row1<fmt, 2>(a, tab);                                                    \
         else gemv_kq_q81_row1<fmt, 4>(a, tab);                                                                 \
     }
-QM_KQ_ROW_KERNEL(qm_gemv_q2k_q81_row, 10)
-QM_KQ_ROW_KERNEL(qm_gemv_iq2xxs_q81_row, 16)
+QM_KQ_ROW_KERNEL(qm_gemv_q2k_q81_row, 10, QM_KQ_ROW_CTAS_Q2K)
+QM_KQ_ROW_KERNEL(qm_gemv_iq2xxs_q81_row, 16, QM_KQ_ROW_CTAS_IQ2XXS)

@@ -870,6 +870,7 @@ int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int3
     // read with direct loads.
     const int64_t row_bytes = (int64_t)w->units * (w->fmt == QM_FMT_Q2_K ? 84 : 66);
     unsigned smem = 0;
+    int64_t resident = 8;   // CTAs of an SM that the grid counts on, by registers (and the table of the IQ2_XXS row kernel)
     if (row_bytes % 16 == 0 && (w->wq & 15) == 0 && qm_env_int("QM_KQ_DIRECT", 0) == 0) {
         // Q8_1 kernels also keep the activations of the CTA's slot in shared memory
         const int64_t xs = xq ? ((int64_t)m * w->units * 8 * 36 + 15) & ~(int64_t)15 : 0;
@@ -879,11 +880,17 @@ int32_t qm_kq_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, bool xq, int3
             ka.xs_bytes = (int32_t)xs;
             smem = (unsigned)(xs + 8 * d * row_bytes);
             // one Q8_1 row: the activations stay in registers up to K = 4096 (6 slots of 2048 x 4096 experts, the layer
-            // of gate, up and down matvecs and its producers: 62.6 -> 57.5 us)
-            if (xq && m == 1 && w->units <= 16) k = w->fmt == QM_FMT_Q2_K ? QM_K_GEMV_Q2K_Q81_ROW : QM_K_GEMV_IQ2XXS_Q81_ROW;
+            // of gate, up and down matvecs and its producers: 62.6 -> 57.5 us). With more CTAs than fit the last ones
+            // start when the rest is done: Q2_K 14336 x 4096, a lone call, 20.5 us at four an SM, 18.4 at three, 18.5 with
+            // the kernel for any m; 8 slots of 1024 x 1024 back to back 6.3, 4.5, 5.9.
+            if (xq && m == 1 && w->units <= 16) {
+                const bool q2k = w->fmt == QM_FMT_Q2_K;
+                k = q2k ? QM_K_GEMV_Q2K_Q81_ROW : QM_K_GEMV_IQ2XXS_Q81_ROW;
+                resident = q2k ? QM_KQ_ROW_CTAS_Q2K : QM_KQ_ROW_CTAS_IQ2XXS;
+            }
         }
     }
-    const int per_sm = smem ? (int)std::max<int64_t>(1, std::min<int64_t>(8, (200 * 1024) / (smem + 3072))) : 8;
+    const int per_sm = smem ? (int)std::max<int64_t>(1, std::min<int64_t>(resident, (200 * 1024) / (smem + 3072))) : 8;
     const int64_t want = (ka.rows + 7) / 8;
     const int64_t cap = std::max<int64_t>(1, (int64_t)c->sm_count * per_sm / std::max(1, slots));
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, cap));

@@ -259,6 +259,10 @@ struct QmCombineArgs {
     int32_t tokens, hidden, topk, pad;
 };
 
+// CTAs of the one-row Q8_1 kernels that fit on an SM by registers (79 and 64 a thread).
+#define QM_KQ_ROW_CTAS_Q2K 3
+#define QM_KQ_ROW_CTAS_IQ2XXS 4
+
 // GEMV over Q2_K / IQ2_XXS weights kept in their GGUF byte layout (qm_gemv_kq.cu).
 struct QmKqArgs {
     const uint8_t *wq;       // [rows][units] super-blocks of 84 (Q2_K) or 66 (IQ2_XXS) bytes; selected form: [experts][rows][units]

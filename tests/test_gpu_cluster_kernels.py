@@ -9,15 +9,15 @@ from lib_b200 import _capi, synth
 from oracle import oracle
 from tests import q8_1_cases as cases
 from tests.capture import launches
+from tests.test_pair_plan import FORMS
 from tests.test_gpu_matmul import TOL as MATMUL_TOL, run as run_matmul
 from tests.test_gpu_stack import build_stack, nre, oracle_chain
 
 pytestmark = pytest.mark.gpu
 
 
-# Rows around one CTA's 128 and a pair's 256; tokens around the rounding to 16, a tile of 32 and the largest tiles;
-# one K unit, fewer units than K shares, more units than the ring of weight items; many row tiles (no split, several
-# rounds per pair).
+# Few rows or tokens, which run as single CTAs with tiles of 32 and 64 tokens: rows around a CTA's 128, tokens around the
+# rounding to 16 and a tile of 32; one K unit, fewer units than K shares, more units than the ring of weight items.
 @pytest.mark.parametrize("n,k,m", [(1, 256, 1), (127, 256, 15), (129, 512, 17), (255, 768, 32), (257, 1024, 33), (256, 2560, 127),
                                    (640, 5120, 129), (272, 256, 255), (520, 512, 257), (144, 2304, 481), (20000, 256, 31),
                                    (9500, 512, 161)])
@@ -25,21 +25,59 @@ def test_matmul_edges(ctx, devbuf, n, k, m):
     assert run_matmul(ctx, devbuf, n, k, m, seed=3 * n + m) <= MATMUL_TOL
 
 
+# Every form of the matmul — pairs and single CTAs, tiles of up to 224 tokens, one to four K shares, several tiles per
+# CTA — with the launch that the plan says. The last 100 rows against the oracle, where the rows are ragged.
+@pytest.mark.parametrize("shape,plan", FORMS)
+def test_matmul_forms(ctx, devbuf, shape, plan):
+    (n, k, m), (cg, bn, splitk, tiles) = shape, plan
+    assert run_matmul(ctx, devbuf, n, k, m, seed=n + m, check_rows=(max(0, n - 100), n)) <= MATMUL_TOL
+    w = ctx.store_create(12, n, k)
+    a, c = devbuf(nbytes=2 * m * k), devbuf(nbytes=4 * m * n)
+    made, = launches(ctx, lambda: ctx.matmul_bf16(w, a.ptr, m, k, c.ptr, n))
+    assert made.name == ("qm_gemm_q4k_pair" if cg == 2 else "qm_gemm_q4k_solo")
+    assert made.grid == cg * (tiles * splitk if splitk > 1 else min(tiles, 148 // cg))
+    w.free()
+
+
 # Two limbs per activation row from three rows on: 14 bits of the unit's maximum, 3e-4 normwise (as in the matvec
-# tests). K of one unit, a partial unit, an odd number of units, and a long K that runs in parts.
+# tests). K of one unit, a partial unit, an odd number of units, and a long K that runs in parts: below the sizes that
+# share a staging.
 @pytest.mark.parametrize("fmt", [2, 8])
 @pytest.mark.parametrize("m", [6, 7, 8])
 @pytest.mark.parametrize("rows,cols,xop", [(16, 256, 0), (33, 288, 1), (2400, 2336, 1), (4736, 1280, 0), (96, 8192, 1)])
-def test_matvec_shared_staging(ctx, devbuf, fmt, m, rows, cols, xop):
+def test_matvec_without_sharing(ctx, devbuf, fmt, m, rows, cols, xop):
     raw = synth.weights(fmt, rows, cols, seed=rows + m)
     w = ctx.store_upload(fmt, rows, cols, raw)
     x = synth.activations(m, cols, 9)
-    yd = devbuf(np.full((m, rows), np.nan, np.float32))
-    ctx.matvec(w, devbuf(x).ptr, m, cols, yd.ptr, rows, xop)
+    xd, yd = devbuf(x), devbuf(np.full((m, rows), np.nan, np.float32))
+    assert not any(k.name.endswith("_x2") for k in launches(ctx, lambda: ctx.matvec(w, xd.ptr, m, cols, yd.ptr, rows, xop)))
+    ctx.matvec(w, xd.ptr, m, cols, yd.ptr, rows, xop)
     got = yd.get((m, rows))
     assert ctx.last_status() == (0, 0)
     want = oracle.MatVec(fmt, raw, rows, cols, oracle.RMSNorm(x) if xop else x)
     assert nre(got, want) <= 3e-4
+    w.free()
+
+
+# Two CTAs share the staging from seven rows and 96 (row, unit) pairs on: the fewest units, a last unit with one block, an
+# odd number of units and the most (one unit less than runs in parts; Q8_0: the most that fit), rows that are no whole
+# tiles and fewer tiles than CTAs, and every input transform (the sums of squares cross the CTAs).
+@pytest.mark.parametrize("fmt,m,rows,cols,xop", [
+    (fmt, m, rows, cols, xop) for fmt in (2, 8) for m in (7, 8) for xop in range(4)
+    for rows, cols in [(33, 3584 if m == 7 else 3072), (2387, 3360), (4737, 4096), (17, 7936 if fmt == 2 else 4096)]])
+def test_matvec_shared_staging(ctx, devbuf, fmt, m, rows, cols, xop):
+    raw = synth.weights(fmt, rows, cols, seed=rows + m)
+    w = ctx.store_upload(fmt, rows, cols, raw)
+    x, x2 = synth.activations(m, cols, 9), synth.activations(m, cols, 10)
+    xd, x2d, yd = devbuf(x), devbuf(x2), devbuf(np.full((m, rows), np.nan, np.float32))
+    call = lambda: ctx.matvec(w, xd.ptr, m, cols, yd.ptr, rows, xop, x2d.ptr if xop >= 2 else 0)
+    assert [k.name[:17] + k.name[-3:] for k in launches(ctx, call)] == ["qm_gemv_q%d0_lean__x2" % (4 if fmt == 2 else 8)]
+    call()
+    got = yd.get((m, rows))
+    assert ctx.last_status() == (0, 0)
+    x64 = x.astype(np.float64)
+    inputs = [x, oracle.RMSNorm(x), oracle.RMSNorm(x + x2), (x64 / (1 + np.exp(-x64)) * x2).astype(np.float32)]
+    assert nre(got, oracle.MatVec(fmt, raw, rows, cols, inputs[xop])) <= 3e-4
     w.free()
 
 
@@ -67,12 +105,32 @@ def test_matvec_that_fits_only_without_sharing(ctx, devbuf, fmt, cols, kernel):
 @pytest.mark.parametrize("hidden,kv,ffn", [(256, 32, 1280), (768, 96, 1792), (1280, 160, 2048)])
 def test_step_shared_staging(ctx, m, hidden, kv, ffn):
     st, raws = build_stack(ctx, 2, hidden, kv, ffn, 12, seed=41)
+    check_step(ctx, st, raws, m, hidden, kv, ffn)
+    st.close()
+
+
+# The kernels whose CTAs share the staging, by their rules on rows and hidden units: one and two column tiles, each number
+# of ring stages, an odd number of units, the down projection whole and in parts; and just below the rules.
+@pytest.mark.parametrize("m,hidden,ffn,kernel", [
+    (4, 3072, 512, "c2d4_x4"), (4, 3328, 1024, "c2d4_x4"), (4, 8192, 512, "c2d3_x4"), (4, 2816, 512, "c2d4"),
+    (5, 2560, 512, "n2d3_x4"), (5, 2304, 512, "n2d3"), (6, 2048, 1024, "n2d3_x4"), (7, 1280, 1280, "n2d3_x4"),
+    (8, 1280, 512, "n2d3_x4"), (8, 1024, 512, "n2d3"), (8, 5120, 512, "n2d2_x4")])
+def test_step_forms(ctx, devbuf, m, hidden, ffn, kernel):
+    kv = 32
+    st, raws = build_stack(ctx, 2 if hidden <= 4096 else 1, hidden, kv, ffn, 12, seed=43)
+    check_step(ctx, st, raws, m, hidden, kv, ffn)
+    xd = devbuf(synth.activations(m, hidden, 8))
+    assert "qm_fused_q4k_dd_" + kernel in [k.name for k in launches(ctx, lambda: st.step(xd.ptr, m, hidden))]
+    st.close()
+
+
+def check_step(ctx, st, raws, m, hidden, kv, ffn):
     x = synth.activations(m, hidden, 8)
     h, kvs = st.step_host(x, want_kv=True)
     want_h, want_kv, _ = oracle_chain(12, raws, x, hidden, kv, ffn)
     assert nre(h, want_h) <= 1e-3 and nre(kvs, want_kv) <= 1e-3
     assert np.array_equal(h, st.step_host(x))
-    st.close()
+    assert ctx.last_status() == (0, 0)
 
 
 # Steps of four super-blocks: a single one, whole steps, a remainder, the largest K in registers and the first beyond.
@@ -93,6 +151,20 @@ def test_q8_1_row(ctx, devbuf, fmt, cols):
     # exact integer sums per group, float32 across groups: 2e-5 of the largest output, as for the other Q8_1 matvecs
     assert np.abs(got[[0, 2]] - want[[0, 2]]).max() <= 2e-5 * np.abs(want[[0, 2]]).max()
     assert np.all(got[1].view(np.uint32) == 0x7fffffff)
+    w.free()
+
+
+# Those kernels hold more registers than the others: a launch starts no more CTAs than run at once.
+@pytest.mark.parametrize("fmt,name,ctas", [(10, "qm_gemv_q2k_q81_row", 3), (16, "qm_gemv_iq2xxs_q81_row", 4)])
+@pytest.mark.parametrize("cols", [1024, 2048, 4096])
+@pytest.mark.parametrize("slots", [1, 8])
+def test_q8_1_row_launch_fits_at_once(ctx, devbuf, fmt, name, ctas, cols, slots):
+    if fmt == 16 and cols == 1024:
+        name, ctas = "qm_gemv_iq2xxs_q81_m1", 8     # rows of 264 bytes: the direct form
+    w = ctx.store_create(fmt, 8 * 14336, cols)
+    b = devbuf(nbytes=4 * 8 * 14336)
+    made, = launches(ctx, lambda: ctx.matvec_selected(w, 8, b.ptr, slots, b.ptr, 0, b.ptr, _capi.FLAG_X_Q8_1))
+    assert made.name == name and 148 * ctas // 2 <= made.grid <= 148 * ctas
     w.free()
 
 
