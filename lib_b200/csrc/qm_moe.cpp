@@ -430,8 +430,10 @@ extern "C" int32_t qm_moe_decode_create(qm_ctx *c, const qm_weight *gate_up, con
         return QM_ERR_SHAPE;
     }
     // One row per op: clusters of four pay only where a warp alone would quantize more than three units of the down
-    // op's x (ffn 14336, 56 units, two tokens: 142 -> 138 us; 11008, 43 units: 118 -> 123; 5632: 123 -> 151).
-    const bool share = max_units >= 50 && c->max_clusters[4] > 0;
+    // op's x (11008, 43 units: 118 -> 123 us; 5632: 123 -> 151). 8 experts, top 2, 1 / 2 / 4 tokens, alone -> shared: hidden
+    // 4096, ffn 14336 (56 units) 83.7 / 140.3 / 256.9 -> 81.5 / 138.8 / 254.5; 3072 x 12800 (50) 72.6 / 118.0 / 218.5 -> 70.3 /
+    // 117.4 / 212.7. One token of hidden 4096 gains from 54 units on (13824: 81.6 -> 79.8; 12800: 75.9 -> 77.3).
+    const bool share = max_units >= (max_tokens == 1 && d->hidden >= 4096 ? 54 : 50) && c->max_clusters[4] > 0;
     d->cluster = share ? 4 : 1;
     d->grid = share ? c->max_clusters[4] * 4 : qm_fused_grid(c);
     d->kernel = (share ? QM_K_DD_X4_SEL_D2 : QM_K_FUSED_Q4K_DD_C4D2_SEL) + (d->plan.depth - 2);

@@ -8,6 +8,7 @@ import pytest
 import lib_b200
 from lib_b200 import synth
 from oracle import oracle
+from tests.capture import launches
 
 pytestmark = pytest.mark.gpu
 
@@ -23,7 +24,8 @@ def chain(gu_raw, dn_raw, hidden, ffn, x, ids, wts):
     return out
 
 
-@pytest.mark.parametrize("experts,hidden,ffn,tokens,topk", [(4, 512, 768, 1, 2), (8, 1024, 1792, 3, 2), (6, 256, 512, 4, 3)])
+@pytest.mark.parametrize("experts,hidden,ffn,tokens,topk", [(4, 512, 768, 1, 2), (8, 1024, 1792, 3, 2), (6, 256, 512, 4, 3),
+                                                              (3, 256, 12800, 1, 2), (2, 512, 14336, 3, 2), (2, 256, 20480, 2, 1)])
 def test_decode_moe_matches_oracle_chain(ctx, devbuf, experts, hidden, ffn, tokens, topk):
     gu_raw = [synth.weights(12, 2 * ffn, hidden, 40 + e) for e in range(experts)]
     dn_raw = [synth.weights(12, hidden, ffn, 140 + e) for e in range(experts)]
@@ -61,6 +63,23 @@ def test_decode_moe_matches_oracle_chain(ctx, devbuf, experts, hidden, ffn, toke
     if tokens > 1:
         assert np.array_equal(got3[1:], got[1:])
     assert ctx.last_status() == (0, 0)
+    ctx.moe_decode_destroy(md)
+    for w in gu + dn:
+        w.free()
+
+
+@pytest.mark.parametrize("hidden,ffn,tokens,kernel", [
+    (256, 12544, 1, "c4d4_sel"), (256, 12800, 1, "c4d4_sel_x4"), (4096, 13568, 1, "c4d4_sel"), (4096, 13568, 2, "c4d4_sel_x4"),
+    (4096, 13824, 1, "c4d4_sel_x4"), (256, 20480, 1, "c4d3_sel_x4")])
+def test_decode_moe_forms(ctx, devbuf, hidden, ffn, tokens, kernel):
+    """Where the CTAs of a cluster share the staging of x, seen from the captured launch."""
+    gu, dn = [ctx.store_create(12, 2 * ffn, hidden)], [ctx.store_create(12, hidden, ffn)]   # (created as zeros)
+    md = ctx.moe_decode_create(gu, dn, 1, tokens)
+    x, ids, wts, out = (devbuf(np.zeros(4 * tokens * hidden, np.uint8)) for _ in range(4))
+    run = lambda: ctx.moe_decode_run(md, x.ptr, tokens, hidden, ids.ptr, wts.ptr, out.ptr, hidden)
+    run()
+    assert ctx.last_status() == (0, 0)
+    assert [k.name for k in launches(ctx, run)] == ["qm_fused_q4k_dd_" + kernel, "qm_moe_decode_combine"]
     ctx.moe_decode_destroy(md)
     for w in gu + dn:
         w.free()
