@@ -2082,7 +2082,6 @@ QM_LEAN_KERNEL(qm_gemv_q80_lean_c2n2d2, 8, 2, 2, 2)
     }
 QM_LEANX_KERNEL(qm_gemv_q40_lean_c2n2d4_x2, 2, 4)
 QM_LEANX_KERNEL(qm_gemv_q40_lean_c2n2d2_x2, 2, 2)
-QM_LEANX_KERNEL(qm_gemv_q80_lean_c2n2d3_x2, 8, 3)
 QM_LEANX_KERNEL(qm_gemv_q80_lean_c2n2d2_x2, 8, 2)
 
 // out[j][r] = c_j * sum over the K parts of a lean matvec, c_j = rsqrt(mean square + eps) from the parts' sums of

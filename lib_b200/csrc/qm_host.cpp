@@ -116,7 +116,7 @@ static const KernelName kKernels[QM_K_COUNT] = {
     {QM_MOD_Q4K, "qm_gemv_q80_lean_c2d2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d3"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2"},
     {QM_MOD_Q4K, "qm_lean_sum"},
     {QM_MOD_Q4K, "qm_gemv_q40_lean_c2n2d4_x2"}, {QM_MOD_Q4K, "qm_gemv_q40_lean_c2n2d2_x2"},
-    {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d3_x2"}, {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2_x2"},
+    {QM_MOD_Q4K, "qm_gemv_q80_lean_c2n2d2_x2"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d3_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_c2d4_x4"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2_x4"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3_x4"},
     {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d2"}, {QM_MOD_Q4K, "qm_fused_q4k_dd_n2d3"},
@@ -946,7 +946,8 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
             if (grid % S != 0) continue;
             if (S > 1 && (!partials || 256 + (int64_t)S * m * ldp * 4 > QM_PARTIALS_BYTES)) continue;
             const int ups = w->units / S;
-            // (shared with the two ring depths, then alone: eight Q8_0 rows of 17 units fit only alone)
+            // (shared with the two ring depths, then alone: eight Q8_0 rows of 17 units fit only alone. Three stages of Q8_0
+            // do not fit beside the seven rows of 14 units that sharing begins with.)
             const int forms = may_share && S == 1 && grid % 2 == 0 ? 4 : 2;
             for (int f = 0; f < forms; f++) {
                 const int share = f < forms - 2 ? 2 : 1, di = f & 1;
@@ -981,7 +982,7 @@ int32_t qm_matvec_launch(qm_ctx *c, const QmWeight *w, uint64_t x_dev, uint64_t 
                     la.ldy = ldp;
                     la.part_stride = (int64_t)m * ldp;
                 }
-                const int k = share == 2 ? (q40 ? QM_K_Q40_LEAN_X2_D4 : QM_K_Q80_LEAN_X2_D3) + di
+                const int k = share == 2 ? (q40 ? QM_K_Q40_LEAN_X2_D4 + di : QM_K_Q80_LEAN_X2_D2)
                                          : (q40 ? QM_K_Q40_LEAN_C4D4 : QM_K_Q80_LEAN_C4D3) + (cpm == 4 ? 0 : nt == 1 ? 2 : 4) + di;
                 int32_t lrc = qm_launch_ex(c, k, (unsigned)grid, 512, (unsigned)smem, &la, true, false, share);
                 if (lrc || S == 1) return lrc;
