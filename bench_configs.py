@@ -313,7 +313,6 @@ def main():
     ap.add_argument("--copies", type=int, default=0, help="weight copies cycled through (default: > L2)")
     ap.add_argument("--iters", type=int, default=20)
     ap.add_argument("--tokens", type=int, default=512)
-    ap.add_argument("--no-pdl", action="store_true")
     ap.add_argument("--exchange", choices=("peer", "nccl"), default="peer", help="config 5 on several GPUs")
     a = ap.parse_args()
     if a.config == 5 and int(os.environ.get("WORLD_SIZE", "1")) > 1:
@@ -321,7 +320,7 @@ def main():
         return
     ctx = lib_b200.Context(0)
     torch.cuda.init()
-    flags = 0 if a.no_pdl else _capi.FLAG_PDL
+    flags = _capi.FLAG_PDL
     out = []
     if a.config == 1:
         out.append(gemv_case(ctx, Q8_0, 4096, 4096, a.m or 1, a.copies, a.iters, flags))

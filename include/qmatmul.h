@@ -185,7 +185,7 @@ QM_API int32_t qm_matvec_selected(qm_ctx *ctx, qm_weight w, int32_t experts, uin
 
 /* Batched / prefill product over a stored Q4_K matrix on the tcgen05 tensor cores:
  * c[j][r] = sum_k a[j][k] * W[r][k] for j < m, a bf16 [m][lda] (16-byte aligned, lda a multiple
- * of 8), c float32 [m][ldc], device pointers. Weights are dequantized into shared memory as
+ * of 8), c float32 [m][ldc], device pointers. Weights are dequantized into tensor memory as
  * bf16, accumulation is fp32 in tensor memory. Supersedes the reference's fp16 wmma prefill
  * GEMM (nvidia/x/cudamoe/prefill.go:97-121). Asynchronous on the context's stream. */
 QM_API int32_t qm_matmul_bf16(qm_ctx *ctx, qm_weight w, uint64_t a_dev, int32_t m, int64_t lda, uint64_t c_dev,
@@ -207,10 +207,12 @@ QM_API int32_t qm_moe_route(qm_ctx *ctx, uint64_t logits_dev, int32_t tokens, in
  * adds a token's expert outputs in slot order. New API of this path: the reference's lm/moe
  * routes and caches experts but has no matmul; its device gather is nvidia/x/cudamoe/moe.go:72-96.
  * All experts run in two grouped launches (gate|up with the SwiGLU in its epilogue, then
- * down); ffn must be a multiple of 128. The list lengths are read back to the host once (one
- * stream synchronization inside the call) to size those launches; with QM_MOE_NOSYNC=1 in the
- * environment nothing is read back and the call is fully asynchronous (slower: the launches
- * then cover the longest possible lists). With QM_MOE_FOLD=1 the gate|up matmul gathers the
+ * down); ffn must be a multiple of 128. An id outside [0, experts) puts its pair into no list:
+ * that slot adds nothing to its token. The list lengths stay on the device and the call is
+ * asynchronous; with QM_MOE_NOSYNC=0 in the environment they are read back once (one stream
+ * synchronization inside the call) to choose the token tile for the longest list, and
+ * QM_MOE_FOLD=1 reads them back unless QM_MOE_NOSYNC=1. Not under stream capture: the call and
+ * qm_moe_experts return CUDA_ERROR_STREAM_CAPTURE_UNSUPPORTED. With QM_MOE_FOLD=1 the gate|up matmul gathers the
  * tokens' rows itself (tile::gather4 copies that follow the dispatch list; needs x 16-byte aligned
  * and ldx a multiple of 8) and no gathered copy is written: the same bits, no 2*pairs*hidden bytes
  * of scratch traffic, but slower on large token tiles. */

@@ -205,7 +205,8 @@ struct QmPairArgs {
     int32_t tiles16;       // 16-row tiles of the store
     int32_t bn;            // tokens per tile, a multiple of 32 up to 256
     int32_t nacc;          // accumulators in tensor memory: 2 where they leave room for four stages (bn <= 128), else 1
-    int32_t stages;        // 128-column stages (A in tensor memory, B in shared memory), 4..8: nacc * bn + 64 * stages <= 512
+    int32_t stages;        // 128-column stages (A in tensor memory, B in shared memory), 2..8 (a single CTA at 224 tokens has 2, at
+                           // 160 and 192 3): nacc * bn + 64 * stages <= 512
     int32_t raw_ring;      // units of weight items in shared memory, 4 to 8
     int32_t box_rows;      // token rows per tile load; a CTA's share of bn is a multiple of it
     int32_t row_tiles;     // tiles of 128 rows per CTA (SwiGLU: 64 gate rows and their up rows)

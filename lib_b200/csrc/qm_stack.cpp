@@ -464,8 +464,8 @@ static int32_t build_fused_dd(qm_ctx *c, qm_stack *s, int m) {
     const bool tp_list = s->tp_world > 1;
     if (m >= qm_env_int("QM_IMAGE_MIN_M", tp_list ? 4 : 9) || qm_env_int("QM_DD", 1) == 0) return QM_ERR_SHAPE;
     // Clusters of four share the staging of x where a CTA alone would quantize about three (row, unit) pairs of the
-    // hidden state per warp; below that their barriers and the 16 SMs they leave idle cost more. Eight layers, alone
-    // -> shared, us: m = 8 hidden 4096 (128 pairs) 796 -> 703, 2048 (64) 456 -> 419, 1280 (40) 440 -> 414; m = 6 4096
+    // hidden state per warp; below that their barriers and the 20 SMs they leave idle cost more (33 clusters of four run at
+    // once, 32 are used: whole clusters in each of the down projection's four groups). Eight layers, alone -> shared, us: m = 8 hidden 4096 (128 pairs) 796 -> 703, 2048 (64) 456 -> 419, 1280 (40) 440 -> 414; m = 6 4096
     // (96) 646 -> 615, 2048 (48) 392 -> 384, 1280 (30) 350 -> 355; m = 5 3072 (60) 441 -> 417, 1280 (25) 325 -> 339;
     // m = 4 4096 (64) 454 -> 420, 3072 (48) 350 -> 345, 2048 (32) 287 -> 304; m = 3 4096 405 -> 400, 1280 slower by a
     // fifth. (Four rows as the barrier form with activation images: 624 at 4096, 401 at 2048, 352 at 1280.)
