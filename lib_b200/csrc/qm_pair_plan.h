@@ -18,7 +18,7 @@ typedef int QmPairClusters[2][5];
 // Estimated cycles: a stage of 128 columns takes 4 cycles per token column on the tensor cores (a CTA alone also copies
 // and reads all of B: 5), at least what its dequantization and hand-over take; a tile's accumulator read-out is hidden
 // by the next tile only where two accumulators fit. The least is set at 500 cycles; time stamps inside the kernel put a
-// stage of 131 to 144 tokens at about 725, with which the formula would take larger tiles for many tokens (256 instead of
+// stage of 160 tokens at about 725, with which the formula would take larger tiles for many tokens (256 instead of
 // 160 for 2048 tokens of 4096 x 4096). Which is faster has not been timed.
 inline QmPairPlan qm_plan_matmul(const QmPairClusters &clusters, int64_t rows, int64_t m, int units) {
     QmPairPlan best = {2, 64, 1, (rows + 255) / 256 * ((m + 63) / 64)};
